@@ -996,7 +996,7 @@ int spl_frame_graph_create(spl_renderer* r, uint32_t width, uint32_t height, uin
         e = cudaGraphGetNodes(g->graph, nullptr, &nn);
         std::vector<cudaGraphNode_t> nodes(nn);
         if (e == cudaSuccess && nn) e = cudaGraphGetNodes(g->graph, nodes.data(), &nn);
-        const void* raster = raster_kernel(r->cfg.use_unaligned_rectangles != 0, r->cfg.blend_mode);
+        const void* raster = raster_kernel(r->cfg.use_unaligned_rectangles != 0, r->cfg.blend_mode, u.margin);
         for (size_t i = 0; e == cudaSuccess && i < nn; ++i) {
             cudaGraphNodeType t;
             if (cudaGraphNodeGetType(nodes[i], &t) != cudaSuccess || t != cudaGraphNodeTypeKernel) continue;

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(256) k_raster_backward(const uint2* __restrict
                             }
                             if (cov) {
                                 const float power = fmaf(tcx, tcx, tcy * tcy);
-                                const float E = spl_expf_nonpos(-0.5f * power);
+                                const float E = spl_expf_falloff<true>(-0.5f * power);
                                 const float a = q1.z;
                                 const float alpha = a * E;
                                 if (!(alpha < alpha_min)) {

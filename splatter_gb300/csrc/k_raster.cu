@@ -302,215 +302,264 @@ __global__ void __launch_bounds__(1024) k_tile_order(const uint2* __restrict__ r
 
 // ------------------------------------------------------------------------------------------------
 constexpr int RASTER_BATCH = 256;
+constexpr int RASTER_WORDS = RASTER_BATCH / 32;
+constexpr float RASTER_NEAR_MARGIN = 9.0f;  // up to this margin a covered pixel's exponent stays above -87
 
 // One CTA per 16x16 tile, one thread per pixel.  Warp w owns the strip of rows 2w, 2w+1; lane l holds
-// column 2 (l / 4) + (l & 1) and row 2w + ((l >> 1) & 1), so the strip's 2x2 blocks are groups of four
-// lanes.  The tile's records (depth order) are staged through shared memory in batches of 256; the
-// thread staging a record also forms its mask of the lanes (pixels) it may draw in each of the eight
-// strips.  Warp-wide bit transposes, four 32-record words at a time, turn its strip's masks into each
-// pixel's list of the batch's records.  The warp then walks the 32 lists of the whole batch at once: in
-// every iteration each pixel takes its next record, so one pass of the per-pixel code serves as many
-// splats as there are lanes with work (most splats here cover a few pixels).  Per pixel: coverage
-// test, falloff, 1/255 discard, blend — the operations of the oracle's raster_tile in the same order,
-// so the image is bit-identical.  Lists are walked in depth order per pixel, a warp whose pixels are
-// all finished skips the rest, and the CTA stops once every pixel is finished (T == 0 in unorm8 mode,
-// T < 1e-4 in fp32 mode).
-// Block indices g (of the eight along a warp's strip) with |c + s g| <= T, widened conservatively:
-// the quotients are clamped to [-1, 9] before rounding outwards, so their float error (a few ulp of
-// at most 9) stays far below the 1e-3 widening.  Empty when lo > hi.
-__device__ __forceinline__ void g_interval(float c, float s, float rs, float T, int& lo, int& hi) {
-    if (fabsf(s) < 1e-30f) {
-        const bool all = fabsf(c) <= T;
-        lo = all ? -1 : 1;
-        hi = all ? 9 : 0;
-        return;
-    }
-    const float q1 = (-T - c) * rs, q2 = (T - c) * rs;  // rs = 1 / s (IEEE: finite, within half an ulp)
-    const float a = fminf(fmaxf(fminf(q1, q2), -1.0f), 9.0f), b = fminf(fmaxf(fmaxf(q1, q2), -1.0f), 9.0f);
-    lo = (int)ceilf(a - 1e-3f);
-    hi = (int)floorf(b + 1e-3f);
+// column l & 15 and row 2w + l / 16.  The tile's records (depth order) are staged through shared memory in batches of 256,
+// last record in slot 0, so that the highest set bit of a list word is its first record; the thread staging a
+// record also forms its mask of the lanes (pixels) it may draw in each of the eight strips.  Warp-wide bit
+// transposes, four 32-record words at a time, turn its strip's masks into each pixel's list of the batch's
+// records, in place.  The warp then walks the 32 lists of the whole batch at once: in every iteration each
+// pixel takes its next record, so one pass of the per-pixel code serves as many splats as there are lanes
+// with work (most splats here cover a few pixels).  Per pixel: coverage test, falloff, 1/255 discard, blend —
+// the operations of the oracle's raster_tile in the same order, so the image is bit-identical.  Lists are
+// walked in depth order per pixel, a warp whose pixels are all finished skips the rest, and the CTA stops
+// once every pixel is finished (T == 0 in unorm8 mode, T < 1e-4 in fp32 mode).
+//
+// Bound by instruction issue (3M splats, 1080p: 78% of issue slots, 192 M warp instructions, DRAM 5%), so the
+// work per list entry and per record is what counts:
+// * lists exact to a pixel row (column interval per row) instead of to a 2x2 block: a walk iteration's lanes
+//   rarely miss the rectangle.  6M splats, 1080p: 400 -> 360 us; 3840x2160: 1,002 -> 924 us;
+// * packed float pairs, the unorm8 target held as k / 255 in floats, no float-to-integer conversions or table
+//   look-ups in the walk, byte permutes and rotations in the transposes, 40 bytes of shared memory read per
+//   list entry instead of 48, two CTA barriers per batch instead of three: 483 -> 400 us; 1,207 -> 1,002 us
+//   (without the packed pairs 417 and 1,062 us).
+// Batches of 512 records (fewer, longer walks) lose more to the fewer resident CTAs: 483 us; five CTAs per
+// SM at 48 registers, without spills: 416 us.
+
+// Two float operations per instruction on packed pairs (the results of the scalar operations, each rounded
+// to nearest).  The assembler contracts a packed product and a packed sum that takes it into a packed fma
+// even where plain contraction is off, so a product that is to be rounded before a sum is a product with a
+// zero addend (fma2, the same value for a non-negative product) or its sum is scalar.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mul.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; add.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{.reg .b64 a, b, c, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mov.b64 c, {%6, %7}; "
+        "fma.rn.f32x2 d, a, b, c; mov.b64 {%0, %1}, d;}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
 }
 
-// Lanes of a warp's 2x16-pixel strip whose column is >= c (0 <= c <= 16); lane l holds column
-// 2 (l / 4) + (l & 1) and row (l >> 1) & 1.
-__device__ __forceinline__ uint32_t strip_columns_from(int c) {
-    const int k = c >> 1;
-    if (c & 1) return (uint32_t)(0xFFFFFFFFull << (4 * k + 4)) | (uint32_t)(0xAull << (4 * k));
-    return (uint32_t)(0xFFFFFFFFull << (4 * k));
+// The unorm8 value nearest to v in [0, 1] (k / 255, k = v * 255 rounded to nearest even), as the float
+// nearest to k / 255: adding 2^23 leaves the integer k in the mantissa's last bits, and k / 255 is the
+// product with the reciprocal's two-float expansion (equal to the correctly rounded quotient for all 256
+// values).  No integer conversions (a quarter of the float rate or less) and no table look-ups.
+__device__ __forceinline__ float2 quantise2(float2 v) {
+    const float2 t = fma2(v, make_float2(255.0f, 255.0f), make_float2(0.0f, 0.0f));
+    const float2 m = add2(t, make_float2(8388608.0f, 8388608.0f));
+    const float2 k = add2(m, make_float2(-8388608.0f, -8388608.0f));
+    const float2 lo = mul2(k, make_float2(UNORM_LO, UNORM_LO));
+    return fma2(k, make_float2(UNORM_HI, UNORM_HI), lo);
 }
 
 // N 32x32 bit-matrix transposes across the warp: afterwards bit i of x[c] in lane l is bit l of the
-// old x[c] in lane i.  Each step d exchanges lane-index bit d with bit-index bit d; the N words go
+// old x[c] in lane i.  Each step d exchanges lane-index bit d with bit-index bit d: whole bytes move by one
+// byte permute for d = 16 and 8, smaller groups by a rotation and one bitwise select.  The N words go
 // through each step together, so their independent shuffle chains overlap their latency (one word
 // at a time, the list building took a quarter of the raster's warp time at 6M splats, 1080p).
 template <int N>
 __device__ __forceinline__ void transpose_lane_bits_n(uint32_t* x, uint32_t lane) {
-    const uint32_t masks[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
+    const uint32_t sel16 = (lane & 16u) ? 0x3276u : 0x5410u, sel8 = (lane & 8u) ? 0x3715u : 0x6240u;
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        const uint32_t d = 16u >> k, m = masks[k];
+    for (int c = 0; c < N; ++c) x[c] = __byte_perm(x[c], __shfl_xor_sync(FULL_MASK, x[c], 16), sel16);
+#pragma unroll
+    for (int c = 0; c < N; ++c) x[c] = __byte_perm(x[c], __shfl_xor_sync(FULL_MASK, x[c], 8), sel8);
+    const uint32_t masks[3] = {0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t d = 4u >> k;
+        const bool up = (lane & d) != 0u;
+        const uint32_t keep = up ? ~masks[k] : masks[k], rot = up ? 32u - d : d;
 #pragma unroll
         for (int c = 0; c < N; ++c) {
             const uint32_t p = __shfl_xor_sync(FULL_MASK, x[c], (int)d);
-            x[c] = (lane & d) ? ((x[c] & ~m) | ((p >> d) & m)) : ((x[c] & m) | ((p & m) << d));
+            x[c] = (x[c] & keep) | (__funnelshift_l(p, p, rot) & ~keep);
         }
     }
 }
 
-template <bool RECT, int BLEND>
+// Highest set bit of x (x != 0).
+__device__ __forceinline__ uint32_t top_bit(uint32_t x) {
+    uint32_t r;
+    asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(x));
+    return r;
+}
+
+// Columns a .. b - 1 of a row of 16 as a bit mask (a, b <= 16, in their low five bits; empty when a >= b).
+__device__ __forceinline__ uint32_t row_columns(uint32_t a, uint32_t b) {
+    return __funnelshift_l(0u, 0xFFFFu, a) & ~__funnelshift_l(0u, 0xFFFFFFFFu, b) & 0xFFFFu;
+}
+
+// FAR: a covered pixel's exponent may fall below -87 (axis-aligned squares, or a margin above
+// RASTER_NEAR_MARGIN), where the falloff takes spl_expf's general path.
+template <bool RECT, int BLEND, bool FAR>
 __global__ void __launch_bounds__(256, 6) k_raster(const uint2* __restrict__ ranges, const uint32_t* __restrict__ tile_order,
                                                 const uint32_t* __restrict__ pair_vals,
                                                 const float4* __restrict__ rec, int W, int H, int tiles_x, float margin,
                                                 float psx, float psy, void* __restrict__ out) {
-    __shared__ float4 s_q0[RASTER_BATCH], s_q1[RASTER_BATCH], s_q2[RASTER_BATCH];
+    // the batch's records, rearranged for packed arithmetic: (A00, A10, A01, A11) (B0, B1, alpha, r) (g, b)
+    __shared__ float4 s_a[RASTER_BATCH], s_b[RASTER_BATCH];
+    __shared__ float2 s_c[RASTER_BATCH];
     __shared__ float4 s_q3[RECT ? 1 : RASTER_BATCH];
-    __shared__ float s_lut[256];
-    __shared__ uint32_t s_pm[8][RASTER_BATCH];             // [strip][record]: lane masks of the batch's records
-    __shared__ uint32_t s_plist[RASTER_BATCH / 32][256];  // [word][pixel]: the pixels' record lists of the batch
+    // [strip][record]: lane masks of the batch's records; then [strip][word * 32 + lane]: the pixels' lists
+    __shared__ uint32_t s_pm[8][RASTER_BATCH];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
-    const uint32_t grp = lane >> 2, li = lane & 3u;
     const int tile = tile_order ? (int)__ldg(tile_order + blockIdx.x) : (int)blockIdx.x;
     const int tx = tile % tiles_x, ty = tile / tiles_x;
-    const int bx0 = tx * TILE_PIXELS + 2 * (int)grp;  // this lane's 2x2 block
-    const int by0 = ty * TILE_PIXELS + 2 * (int)w;
-    const int px = bx0 + (int)(li & 1u), py = by0 + (int)(li >> 1);
+    const int wx0 = tx * TILE_PIXELS;
+    const int px = wx0 + (int)(lane & 15u), py = ty * TILE_PIXELS + 2 * (int)w + (int)(lane >> 4);
     const float X = (float)px + 0.5f, Y = (float)py + 0.5f;
-    s_lut[tid] = (float)tid / 255.0f;
     const uint2 rg = ranges[tile];
     const bool inside = px < W && py < H;
     bool done = !inside;
     bool warp_done = __all_sync(FULL_MASK, done);
-    int cr = 0, cg = 0, cb = 0, ta = 255;
-    float fr = 0.0f, fg = 0.0f, fb = 0.0f, ft = 1.0f;
+    // (r, g) and (b, T): unorm8 values as floats k / 255, or the fp32 target
+    float2 rgv = make_float2(0.0f, 0.0f), bt = make_float2(0.0f, 1.0f);
     const float alpha_min = 1.0f / 255.0f;
-    const int wx0 = tx * TILE_PIXELS;  // the eight blocks of this warp: columns wx0 + 2g, + 1, rows by0, by0+1
     for (uint32_t b = rg.x; b < rg.y; b += RASTER_BATCH) {
-        __syncthreads();
-        const uint32_t i = b + tid;
-        if (i < rg.y) {
-            const uint32_t slot = __ldg(pair_vals + i);
-            const float4* r = rec + (size_t)slot * 4;
-            const float4 r0 = __ldg(r + 0), r1 = __ldg(r + 1), r2 = __ldg(r + 2);
-            s_q0[tid] = r0;
-            s_q1[tid] = r1;
-            s_q2[tid] = r2;
-            if (!RECT) s_q3[tid] = __ldg(r + 3);
-            // The record's lane mask for each of the tile's eight strips (rows 2w, 2w + 1): the pixels
-            // inside its pixel box and, for rectangles, only in the 2x2 blocks where some pixel
-            // centre may lie in the rectangle: over a block's four centres tc lies within tc(block
-            // centre) +- ext (half the block's extent mapped by |A|, widened by a rounding bound far
-            // above the per-pixel FMA chains' error), and along the strip the block centre's tc is
-            // c + 2g A, so |c + 2g A| <= margin + ext is an interval of block indices g.  Skipped
-            // pixels are not drawn by the record: the image is unchanged.
+        const uint32_t i = b + tid, slot = RASTER_BATCH - 1u - tid;
 #pragma unroll
-            for (int sw = 0; sw < 8; ++sw) s_pm[sw][tid] = 0u;
+        for (int sw = 0; sw < 8; ++sw) s_pm[sw][slot] = 0u;
+        if (i < rg.y) {
+            const uint32_t rs = __ldg(pair_vals + i);
+            const float4* r = rec + (size_t)rs * 4;
+            const float4 r0 = __ldg(r + 0), r1 = __ldg(r + 1), r2 = __ldg(r + 2);
+            s_a[slot] = make_float4(r0.x, r0.w, r0.y, r1.x);
+            s_b[slot] = make_float4(r0.z, r1.y, r1.z, r2.x);
+            s_c[slot] = make_float2(r2.y, r2.z);
+            if (!RECT) s_q3[slot] = __ldg(r + 3);
+            // The record's lane mask for each of the tile's eight strips (rows 2w, 2w + 1), one 16-bit half
+            // per row: the pixels inside its pixel box and, for rectangles, only those whose centre may lie in
+            // the rectangle: along a row tc is c + x A, so |c + x A| <= T is the interval (-c +- T) / A of
+            // columns x.  T is the margin widened by a rounding bound far above the errors of the
+            // per-pixel FMA chains and of this arithmetic (1e-6 of each term of c and of T itself), the
+            // interval by another 1e-3 columns.  Pixels left out are not drawn by the record: the image
+            // is unchanged.
             const uint32_t lo = __float_as_uint(r1.w), hi = __float_as_uint(r2.w);
             const int x0 = (int)(lo & 0xFFFFu), y0 = (int)(lo >> 16);
             const int x1 = (int)(hi & 0xFFFFu), y1 = (int)(hi >> 16);
             if (x0 <= x1 && y0 <= y1) {
                 const int ty0 = ty * TILE_PIXELS;
-                const int sw0 = max((y0 - ty0) >> 1, 0), sw1 = min((y1 - ty0) >> 1, 7);  // floor halves
-                float rsx = 0.0f, rsy = 0.0f;
+                const int ra = max(y0 - ty0, 0), rb = min(y1 - ty0, 15);  // the box's rows and columns here
+                const uint32_t box = row_columns((uint32_t)max(x0 - wx0, 0), (uint32_t)min(x1 - wx0, 15) + 1u);
+                float2 c = make_float2(0.0f, 0.0f), step = c, half = make_float2(1e9f, 1e9f);
                 if (RECT) {
-                    rsx = 1.0f / (2.0f * r0.x);
-                    rsy = 1.0f / (2.0f * r0.w);
+                    // column 0 of row ra; row after row the interval's centre moves by step
+                    const float Xc = (float)wx0 + 0.5f, Yc = (float)(ty0 + ra) + 0.5f;
+                    const float Xm = (float)(wx0 + 16), Ym = (float)(ty0 + 16);
+                    if (fabsf(r0.x) > 1e-30f) {
+                        const float s = -1.0f / r0.x;
+                        const float T = margin + 1e-6f * (fabsf(r0.x) * Xm + fabsf(r0.y) * Ym + fabsf(r0.z) + margin);
+                        c.x = fmaf(r0.y, Yc, fmaf(r0.x, Xc, r0.z)) * s;
+                        step.x = r0.y * s;
+                        half.x = T * fabsf(s) + 1e-3f;
+                    }
+                    if (fabsf(r0.w) > 1e-30f) {
+                        const float s = -1.0f / r0.w;
+                        const float T = margin + 1e-6f * (fabsf(r0.w) * Xm + fabsf(r1.x) * Ym + fabsf(r1.y) + margin);
+                        c.y = fmaf(r1.x, Yc, fmaf(r0.w, Xc, r1.y)) * s;
+                        step.y = r1.x * s;
+                        half.y = T * fabsf(s) + 1e-3f;
+                    }
                 }
-                for (int sw = sw0; sw <= sw1; ++sw) {
-                    const int sy0 = ty0 + 2 * sw;  // the strip's first row
-                    int ca = x0 - wx0, cb = x1 - wx0;  // strip columns of the box
+                uint16_t* pm = reinterpret_cast<uint16_t*>(&s_pm[0][slot]);
+                for (int row = ra; row <= rb; ++row) {
+                    uint32_t m = box;
                     if (RECT) {
-                        const float Xc = (float)(wx0 + 1), Yc = (float)(sy0 + 1);  // block 0's centre
-                        const float Xm = (float)(wx0 + 16), Ym = (float)(sy0 + 2);
-                        const float cx = fmaf(r0.y, Yc, fmaf(r0.x, Xc, r0.z));
-                        const float cy = fmaf(r1.x, Yc, fmaf(r0.w, Xc, r1.y));
-                        const float Tx = margin + 0.5f * (fabsf(r0.x) + fabsf(r0.y)) +
-                                         1e-6f * (fabsf(r0.x) * Xm + fabsf(r0.y) * Ym + fabsf(r0.z));
-                        const float Ty = margin + 0.5f * (fabsf(r0.w) + fabsf(r1.x)) +
-                                         1e-6f * (fabsf(r0.w) * Xm + fabsf(r1.x) * Ym + fabsf(r1.y));
-                        int lx, hx, ly, hy;
-                        g_interval(cx, 2.0f * r0.x, rsx, Tx, lx, hx);
-                        g_interval(cy, 2.0f * r0.w, rsy, Ty, ly, hy);
-                        ca = max(ca, 2 * max(lx, ly));
-                        cb = min(cb, 2 * min(hx, hy) + 1);
+                        const float k = (float)(row - ra);
+                        const float2 q = fma2(make_float2(k, k), step, c);
+                        const float2 qa = add2(q, make_float2(-half.x, -half.y)), qb = add2(q, half);
+                        // first column: the bound rounded up; one past the last: rounded down, plus one
+                        const float fa = fminf(fmaxf(fmaxf(qa.x, qa.y), 0.0f), 16.0f);
+                        const float fb = fmaxf(fminf(fminf(qb.x, qb.y), 15.0f), -1.0f);
+                        m &= row_columns(__float_as_uint(__fadd_ru(fa, 8388608.0f)),
+                                         __float_as_uint(__fadd_rd(fb, 8388609.0f)));
                     }
-                    ca = max(ca, 0);
-                    cb = min(cb, 15);
-                    if (ca <= cb) {
-                        uint32_t pm = strip_columns_from(ca) & ~strip_columns_from(cb + 1);
-                        if (y0 > sy0) pm &= 0xCCCCCCCCu;      // lanes of the strip's second row
-                        if (y1 < sy0 + 1) pm &= 0x33333333u;  // lanes of its first row
-                        s_pm[sw][tid] = pm;
-                    }
+                    // strip row / 2, half row & 1
+                    pm[(row >> 1) * (2 * RASTER_BATCH) + (row & 1)] = (uint16_t)m;
                 }
             }
         }
         __syncthreads();
-        const uint32_t cnt = min((uint32_t)RASTER_BATCH, rg.y - b);
         if (!warp_done) {
-            // Per-pixel lists of the batch, 32 records per step: the strip's lane masks of records
-            // 32c + l, transposed so that lane p holds word c of pixel p's list (bit i: record 32c + i),
-            // kept in s_plist; bit c of `nz` marks a non-empty word.
+            // Per-pixel lists of the batch: the strip's lane masks of slots 32c + l, transposed so that lane p
+            // holds word c of pixel p's list (bit i: slot 32c + i); bit c of `nz` marks a non-empty word.
             uint32_t nz = 0u;
-            uint32_t t[RASTER_BATCH / 32];
 #pragma unroll
-            for (int c = 0; c < RASTER_BATCH / 32; ++c) {
-                const uint32_t jl = (uint32_t)c * 32u + lane;
-                t[c] = jl < cnt ? s_pm[w][jl] : 0u;
-            }
-            // four words at a time; a group whose 128 records miss the strip stays zero
-            if (__any_sync(FULL_MASK, ((t[0] | t[1]) | (t[2] | t[3])) != 0u)) transpose_lane_bits_n<4>(t, lane);
-            if (cnt > 128u && __any_sync(FULL_MASK, ((t[4] | t[5]) | (t[6] | t[7])) != 0u))
-                transpose_lane_bits_n<4>(t + 4, lane);
+            for (int c0 = 0; c0 < RASTER_WORDS; c0 += 4) {
+                uint32_t t[4];
 #pragma unroll
-            for (int c = 0; c < RASTER_BATCH / 32; ++c) {
-                s_plist[c][tid] = t[c];
-                nz |= (t[c] != 0u ? 1u : 0u) << c;
+                for (int c = 0; c < 4; ++c) t[c] = s_pm[w][(c0 + c) * 32 + lane];
+                // a group whose 128 records miss the strip stays zero
+                if (__any_sync(FULL_MASK, ((t[0] | t[1]) | (t[2] | t[3])) != 0u)) {
+                    transpose_lane_bits_n<4>(t, lane);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        s_pm[w][(c0 + c) * 32 + lane] = t[c];
+                        nz |= (t[c] != 0u ? 1u : 0u) << (c0 + c);
+                    }
+                }
             }
             // Walk the 32 lists at once across the whole batch: in every iteration each pixel takes its
             // next record.  The warp leaves once every pixel is finished or has walked its list.
+            if (done) nz = 0u;
             uint32_t cur = 0u, cbase = 0u;
             while (true) {
                 if (cur == 0u && nz != 0u) {
-                    const uint32_t c = (uint32_t)(__ffs(nz) - 1);
-                    nz &= nz - 1u;
-                    cur = s_plist[c][tid];
+                    const uint32_t c = top_bit(nz);
+                    nz ^= 1u << c;
                     cbase = c * 32u;
+                    cur = s_pm[w][cbase + lane];
                 }
-                if (!__any_sync(FULL_MASK, cur != 0u && !done)) break;
-                if (cur == 0u || done) continue;
-                const uint32_t j = cbase + (uint32_t)(__ffs(cur) - 1);
-                cur &= cur - 1u;
-                const float4 q1 = s_q1[j], q2 = s_q2[j];
-                const float4 q0 = s_q0[j];
-                const float tcx = fmaf(q0.y, Y, fmaf(q0.x, X, q0.z));
-                const float tcy = fmaf(q1.x, Y, fmaf(q0.w, X, q1.y));
+                if (!__any_sync(FULL_MASK, cur != 0u)) break;
+                if (cur == 0u) continue;
+                const uint32_t bit = top_bit(cur);
+                const uint32_t j = cbase + bit;
+                cur ^= 1u << bit;
+                const float4 qa = s_a[j], qb = s_b[j];
+                const float2 tc = fma2(make_float2(qa.z, qa.w), make_float2(Y, Y),
+                                       fma2(make_float2(qa.x, qa.y), make_float2(X, X), make_float2(qb.x, qb.y)));
                 if (RECT) {
-                    if (!(fabsf(tcx) <= margin && fabsf(tcy) <= margin)) continue;
+                    if (!(fabsf(tc.x) <= margin && fabsf(tc.y) <= margin)) continue;
                 } else {
                     const float4 q3 = s_q3[j];
                     const float dx = fmaf(psx, X, q3.x), dy = fmaf(psy, Y, q3.y);
                     if (!(fabsf(dx) <= q3.z && fabsf(dy) <= q3.z)) continue;
                 }
-                const float power = fmaf(tcx, tcx, tcy * tcy);
-                const float alpha = q1.z * spl_expf_nonpos(-0.5f * power);
+                const float power = fmaf(tc.x, tc.x, tc.y * tc.y);
+                const float alpha = qb.z * spl_expf_falloff<FAR>(-0.5f * power);
                 if (alpha < alpha_min) continue;
-                // __saturatef == clamp to [0, 1] (NaN -> 0); __float2int_rn == (int)rintf
-                const float sr = __saturatef(q2.x * alpha), sg = __saturatef(q2.y * alpha);
-                const float sb = __saturatef(q2.z * alpha), sa = __saturatef(alpha);
+                const float2 qc = s_c[j];
+                // __saturatef == clamp to [0, 1] (NaN -> 0)
+                const float sr = __saturatef(qb.w * alpha), sg = __saturatef(qc.x * alpha);
+                const float sb = __saturatef(qc.y * alpha), om = 1.0f - __saturatef(alpha);
+                const float2 TT = make_float2(bt.y, bt.y);
+                const float2 u = mul2(make_float2(sr, sg), TT), v = mul2(make_float2(sb, om), TT);
                 if (BLEND == 0) {
-                    const float dA = s_lut[ta];
-                    cr = __float2int_rn(__saturatef(sr * dA + s_lut[cr]) * 255.0f);
-                    cg = __float2int_rn(__saturatef(sg * dA + s_lut[cg]) * 255.0f);
-                    cb = __float2int_rn(__saturatef(sb * dA + s_lut[cb]) * 255.0f);
-                    ta = __float2int_rn(__saturatef(dA * (1.0f - sa)) * 255.0f);
-                    done = ta == 0;
+                    rgv = quantise2(make_float2(__saturatef(u.x + rgv.x), __saturatef(u.y + rgv.y)));
+                    bt = quantise2(make_float2(__saturatef(v.x + bt.x), v.y));
+                    done = bt.y == 0.0f;
                 } else {
-                    fr = sr * ft + fr;
-                    fg = sg * ft + fg;
-                    fb = sb * ft + fb;
-                    ft = ft * (1.0f - sa);
-                    done = ft < FP32_T_MIN;
+                    rgv = make_float2(u.x + rgv.x, u.y + rgv.y);
+                    bt = make_float2(v.x + bt.x, v.y);
+                    done = bt.y < FP32_T_MIN;
                 }
+                if (done) cur = nz = 0u;
             }
             warp_done = __all_sync(FULL_MASK, done);
         }
@@ -519,19 +568,24 @@ __global__ void __launch_bounds__(256, 6) k_raster(const uint2* __restrict__ ran
     if (inside) {
         const size_t pix = (size_t)py * (size_t)W + (size_t)px;
         if (BLEND == 0) {
-            reinterpret_cast<uchar4*>(out)[pix] = make_uchar4((unsigned char)cr, (unsigned char)cg, (unsigned char)cb,
-                                                              (unsigned char)ta);
+            const auto byte = [](float v) { return (unsigned char)__float2int_rn(v * 255.0f); };
+            reinterpret_cast<uchar4*>(out)[pix] = make_uchar4(byte(rgv.x), byte(rgv.y), byte(bt.x), byte(bt.y));
         } else {
-            reinterpret_cast<float4*>(out)[pix] = make_float4(fr, fg, fb, ft);
+            reinterpret_cast<float4*>(out)[pix] = make_float4(rgv.x, rgv.y, bt.x, bt.y);
         }
     }
 }
 
-const void* raster_kernel(bool rect, int blend) {
-    if (rect) return blend == 0 ? reinterpret_cast<const void*>(&k_raster<true, 0>)
-                                : reinterpret_cast<const void*>(&k_raster<true, 1>);
-    return blend == 0 ? reinterpret_cast<const void*>(&k_raster<false, 0>)
-                      : reinterpret_cast<const void*>(&k_raster<false, 1>);
+typedef void (*RasterKernel)(const uint2*, const uint32_t*, const uint32_t*, const float4*, int, int, int, float,
+                             float, float, void*);
+static RasterKernel pick_raster(bool rect, int blend, float margin) {
+    if (!rect) return blend == 0 ? k_raster<false, 0, true> : k_raster<false, 1, true>;
+    if (fabsf(margin) <= RASTER_NEAR_MARGIN) return blend == 0 ? k_raster<true, 0, false> : k_raster<true, 1, false>;
+    return blend == 0 ? k_raster<true, 0, true> : k_raster<true, 1, true>;
+}
+
+const void* raster_kernel(bool rect, int blend, float margin) {
+    return reinterpret_cast<const void*>(pick_raster(rect, blend, margin));
 }
 
 void launch_raster(bool rect, int blend, const uint2* ranges, uint32_t* tile_order, const uint32_t* pair_vals,
@@ -543,18 +597,8 @@ void launch_raster(bool rect, int blend, const uint2* ranges, uint32_t* tile_ord
     const float psx = (2.0f * u.view_size[0]) / (float)W;
     const float psy = -((2.0f * u.view_size[1]) / (float)H);
     if (tile_order) k_tile_order<<<1, 1024, 0, st>>>(ranges, (uint32_t)grid, tile_order);
-    const uint32_t* o = tile_order;
-    if (rect) {
-        if (blend == 0)
-            k_raster<true, 0><<<grid, 256, 0, st>>>(ranges, o, pair_vals, rec, W, H, tiles_x, u.margin, psx, psy, out);
-        else
-            k_raster<true, 1><<<grid, 256, 0, st>>>(ranges, o, pair_vals, rec, W, H, tiles_x, u.margin, psx, psy, out);
-    } else {
-        if (blend == 0)
-            k_raster<false, 0><<<grid, 256, 0, st>>>(ranges, o, pair_vals, rec, W, H, tiles_x, u.margin, psx, psy, out);
-        else
-            k_raster<false, 1><<<grid, 256, 0, st>>>(ranges, o, pair_vals, rec, W, H, tiles_x, u.margin, psx, psy, out);
-    }
+    pick_raster(rect, blend, u.margin)<<<grid, 256, 0, st>>>(ranges, tile_order, pair_vals, rec, W, H, tiles_x, u.margin,
+                                                             psx, psy, out);
 }
 
 }  // namespace spl

@@ -132,11 +132,15 @@ __device__ __forceinline__ float spl_expf(float x) {
     return __fmul_rn(__fmul_rn(p, s1), s2);
 }
 
-// spl_expf restricted to finite x <= 0 (the fragment falloff): the same result bit for bit.  For
-// n >= -125 the two-factor scaling reduces to one multiply by 2^n, exact because p * 2^n is normal.
-__device__ __forceinline__ float spl_expf_nonpos(float x) {
-    if (x < -87.0f) return spl_expf(x);
-    const float n = rintf(__fmul_rn(x, 1.44269502162933349609375f));
+// spl_expf restricted to finite x <= 0 (the fragment falloff): the same result bit for bit.  Adding
+// 1.5 x 2^23 rounds x log2(e) to the nearest integer n, ties to even as rintf does, and leaves n in the
+// sum's low bits, so that the scaling by 2^n (p 2^n is normal for n >= -125) is one integer shift-add and no
+// float-to-integer conversion is needed.  FAR: x may lie below -87 (or be NaN), the general path's case.
+template <bool FAR>
+__device__ __forceinline__ float spl_expf_falloff(float x) {
+    if (FAR && !(x >= -87.0f)) return spl_expf(x);
+    const float m = __fadd_rn(__fmul_rn(x, 1.44269502162933349609375f), 12582912.0f);
+    const float n = m - 12582912.0f;
     float r = fmaf(n, -0.693145751953125f, x);
     r = fmaf(n, -1.428606765330187045e-06f, r);
     float p = 1.98412698412698412e-04f;
@@ -147,8 +151,12 @@ __device__ __forceinline__ float spl_expf_nonpos(float x) {
     p = fmaf(p, r, 0.5f);
     p = fmaf(p, r, 1.0f);
     p = fmaf(p, r, 1.0f);
-    return __fmul_rn(p, __int_as_float(((int)n + 127) << 23));
+    return __uint_as_float(__float_as_uint(p) + (__float_as_uint(m) << 23));
 }
+
+// 1/255 as a sum of two floats: k UNORM_HI + (k UNORM_LO rounded), in one fma, is k / 255 correctly rounded
+// for k = 0 .. 255.
+constexpr float UNORM_HI = 0x1.010102p-8f, UNORM_LO = -0x1.fdfdfep-33f;
 
 // The loader's transform of one splat (Scene::load_chunk, scene.rs:225-250): quaternion normalised,
 // log-scales clamped to their mean +- 5 and exponentiated, opacity logit through the sigmoid.
