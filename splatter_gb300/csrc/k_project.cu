@@ -204,43 +204,84 @@ void launch_cull_key(int mode, bool hist, uint32_t grid_n, const SceneView* d_sv
 }
 
 // ------------------------------------------------------------------------------------------------
-template <int SHO>
-__device__ __forceinline__ void load_sh(const float* __restrict__ sh, uint32_t i, float* out) {
-    constexpr int NF = 3 * (SHO + 1) * (SHO + 1);
-    constexpr int NV = (NF + 3) / 4;
-    const float4* p = reinterpret_cast<const float4*>(sh + (size_t)i * 48);
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        const float4 v = __ldg(p + k);
-        out[4 * k + 0] = v.x;
-        if (4 * k + 1 < 48) out[4 * k + 1] = v.y;
-        if (4 * k + 2 < 48) out[4 * k + 2] = v.z;
-        if (4 * k + 3 < 48) out[4 * k + 3] = v.w;
-    }
-}
+// Vertex stage, a warp for 32 visible splats at a time.  STAGED: their SH rows (NV 16-byte pieces of the
+// 192-byte rows) come through shared memory: lane l of load k copies piece (32 k + l) of the warp's 32 NV
+// pieces, so that a load's lanes cover whole rows.  One row per lane instead touches 32 different 128-byte
+// lines with every load, and the L1's line accesses bound the kernel (78% of their peak, 408 per warp of 32
+// splats).  The copies are asynchronous: the shape is computed while they are in flight.  6M splats, SH 3,
+// 4.33M visible: 246 -> 219 us, 91% of the copy bandwidth on 312 bytes per visible splat (seven CTAs of four
+// warps per SM at 72 registers; six 223 us; eight 219 us, but slower than seven below 1M splats; a grid of the
+// resident CTAs alone 228 us).  Where one wave of warps holds all splats the detour only adds latency (frames
+// of 2k, 100k and 350k splats 0.8-1.2 us longer, 1M splats 1.1 us shorter): below PRE_STAGED_MIN splats,
+// and for degree 0, whose rows are one piece, each lane reads its own row.
+constexpr uint32_t PRE_STAGED_MIN = 1u << 19;
 
-template <int SHO, bool COV, bool RECT>
-__global__ void __launch_bounds__(256) k_preprocess(const SceneView* __restrict__ d_sv,
+template <int SHO, bool STAGED>
+struct PreShape {
+    static constexpr int NV = (3 * (SHO + 1) * (SHO + 1) + 3) / 4;  // 1, 3, 7 or 12 pieces of a row
+    static constexpr int STRIDE = NV | 1;  // in shared memory, odd: a lane per row reads without bank conflicts
+    static constexpr int WARPS = STAGED ? 4 : 8, CTAS = STAGED ? 7 : 3;
+};
+
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <int SHO, bool COV, bool RECT, bool STAGED>
+__global__ void __launch_bounds__(PreShape<SHO, STAGED>::WARPS * 32, PreShape<SHO, STAGED>::CTAS) k_preprocess(const SceneView* __restrict__ d_sv,
                                                     const Uniforms* __restrict__ d_u,
                                                     const uint32_t* __restrict__ idx,
                                                     const FrameCounters* __restrict__ fc, float4* __restrict__ rec,
                                                     uint2* __restrict__ boxes) {
+    constexpr int NV = PreShape<SHO, STAGED>::NV, STRIDE = PreShape<SHO, STAGED>::STRIDE;
+    __shared__ float4 s_sh[PreShape<SHO, STAGED>::WARPS][STAGED ? 32 * STRIDE : 1];
     __shared__ Uniforms s_u;
     __shared__ SceneView s_sv;
     stage_frame(d_u, s_u, d_sv, s_sv);
     __syncthreads();
     const Uniforms& u = s_u;
     const SceneView& s = s_sv;
-    const uint32_t V = fc->visible;
-    for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < V; slot += gridDim.x * blockDim.x) {
-        const uint32_t i = __ldg(idx + slot);
-        const float cx = __ldg(s.x + i), cy = __ldg(s.y + i), cz = __ldg(s.z + i);
-        const float4 rot = __ldg(s.rot + i);
-        const float4 sca = __ldg(s.scale_alpha + i);
-        float sh[48];
-        load_sh<SHO>(s.sh, i, sh);
-        VertexOut<float> o;
-        vertex_math<SHO, COV, float>(u, cx, cy, cz, rot.x, rot.y, rot.z, rot.w, sca.x, sca.y, sca.z, sh, o);
+    const uint32_t V = fc->visible, lane = threadIdx.x & 31u;
+    float4* rows = s_sh[threadIdx.x >> 5];
+    const uint32_t step = gridDim.x * blockDim.x;
+    uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t i = STAGED && slot < V ? __ldg(idx + slot) : 0u;
+    for (; slot - lane < V; slot += step) {  // the warp's 32 slots; lanes past V only help to copy
+        const uint32_t live = min(32u, V - (slot - lane));
+        if constexpr (STAGED) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                const uint32_t piece = 32u * k + lane, row = piece / NV, col = piece - row * NV;
+                const uint32_t ir = __shfl_sync(FULL_MASK, i, (int)row);
+                if (row < live) copy16_async(rows + row * STRIDE + col, s.sh + (size_t)ir * 48 + col * 4);
+            }
+        } else {
+            if (slot >= V) break;
+            i = __ldg(idx + slot);
+        }
+        const bool mine = !STAGED || lane < live;
+        float cx = 0.0f, cy = 0.0f, cz = 0.0f;
+        float4 rot = make_float4(0.0f, 0.0f, 0.0f, 0.0f), sca = rot;
+        float c[3];
+        if (mine) {
+            cx = __ldg(s.x + i);
+            cy = __ldg(s.y + i);
+            cz = __ldg(s.z + i);
+            rot = __ldg(s.rot + i);
+            sca = __ldg(s.scale_alpha + i);
+        }
+        if constexpr (!STAGED) {
+            float4 row[NV];
+            const float4* r = reinterpret_cast<const float4*>(s.sh + (size_t)i * 48);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) row[k] = __ldg(r + k);
+            vertex_colour<SHO, STAGED>(u, cx, cy, cz, row, c);
+        }
+        if (STAGED) i = slot + step < V ? __ldg(idx + slot + step) : 0u;  // the next iteration's splat
+        VertexShape<float> o;
+        vertex_shape<COV, float>(u, cx, cy, cz, rot.x, rot.y, rot.z, rot.w, sca.x, sca.y, sca.z, o);
         // pixel box of the rectangle (or AA square) and validity
         const float vw = u.view_size[0], vh = u.view_size[1];
         const float Wf = (float)u.image_size[0], Hf = (float)u.image_size[1];
@@ -262,8 +303,14 @@ __global__ void __launch_bounds__(256) k_preprocess(const SceneView* __restrict_
         const float fx0 = ceilf(((cxp - exq) - eps) - 0.5f), fx1 = floorf(((cxp + exq) + eps) - 0.5f);
         const float fy0 = ceilf(((cyp - eyq) - eps) - 0.5f), fy1 = floorf(((cyp + eyq) + eps) - 0.5f);
         const float al = sca.w;
+        if constexpr (STAGED) {
+            wait_copies();
+            __syncwarp();
+            vertex_colour<SHO, STAGED>(u, cx, cy, cz, rows + lane * STRIDE, c);
+            __syncwarp();  // the rows are read before the next iteration's copies
+        }
         bool ok = isfinite(o.A00) && isfinite(o.A01) && isfinite(o.B0) && isfinite(o.A10) && isfinite(o.A11) &&
-                  isfinite(o.B1) && isfinite(o.cr) && isfinite(o.cg) && isfinite(o.cb) && isfinite(fx0) &&
+                  isfinite(o.B1) && isfinite(c[0]) && isfinite(c[1]) && isfinite(c[2]) && isfinite(fx0) &&
                   isfinite(fx1) && isfinite(fy0) && isfinite(fy1) && isfinite(R) && isfinite(o.bx) && isfinite(o.by) &&
                   (al >= 1.0f / 255.0f);
         uint32_t lo = 0xFFFFFFFFu, hi = 0u;
@@ -275,45 +322,43 @@ __global__ void __launch_bounds__(256) k_preprocess(const SceneView* __restrict_
                 hi = (uint32_t)(int)cx1 | ((uint32_t)(int)cy1 << 16);
             }
         }
-        float4* q = rec + (size_t)slot * 4;
-        q[0] = make_float4(o.A00, o.A01, o.B0, o.A10);
-        q[1] = make_float4(o.A11, o.B1, al, __uint_as_float(lo));
-        q[2] = make_float4(o.cr, o.cg, o.cb, __uint_as_float(hi));
-        q[3] = RECT ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : make_float4(o.bx, o.by, R, 0.0f);
-        boxes[slot] = make_uint2(lo, hi);  // compact copy for the binning kernel
+        if (mine) {
+            float4* q = rec + (size_t)slot * 4;
+            q[0] = make_float4(o.A00, o.A01, o.B0, o.A10);
+            q[1] = make_float4(o.A11, o.B1, al, __uint_as_float(lo));
+            q[2] = make_float4(c[0], c[1], c[2], __uint_as_float(hi));
+            q[3] = RECT ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : make_float4(o.bx, o.by, R, 0.0f);
+            boxes[slot] = make_uint2(lo, hi);  // compact copy for the binning kernel
+        }
     }
 }
 
-template <int SHO, bool COV>
-static void launch_pre2(bool rect, dim3 g, const SceneView* s, const Uniforms* u, const uint32_t* idx,
-                        const FrameCounters* fc, float4* rec, uint2* boxes, cudaStream_t st) {
-    if (rect)
-        k_preprocess<SHO, COV, true><<<g, 256, 0, st>>>(s, u, idx, fc, rec, boxes);
-    else
-        k_preprocess<SHO, COV, false><<<g, 256, 0, st>>>(s, u, idx, fc, rec, boxes);
+template <int SHO, bool COV, bool RECT, bool STAGED>
+static void launch_pre3(const SceneView* s, const Uniforms* u, const uint32_t* idx, const FrameCounters* fc, float4* rec,
+                        uint2* boxes, uint32_t max_n, cudaStream_t st) {
+    constexpr uint32_t threads = PreShape<SHO, STAGED>::WARPS * 32;
+    // grid stride beyond 4096 threads per SM
+    const uint32_t blocks = (max_n + threads - 1) / threads, cap = device_sm_count() * (4096u / threads);
+    k_preprocess<SHO, COV, RECT, STAGED><<<blocks < cap ? blocks : cap, threads, 0, st>>>(s, u, idx, fc, rec, boxes);
 }
 template <int SHO>
-static void launch_pre1(bool cov, bool rect, dim3 g, const SceneView* s, const Uniforms* u, const uint32_t* idx,
-                        const FrameCounters* fc, float4* rec, uint2* boxes, cudaStream_t st) {
-    if (cov)
-        launch_pre2<SHO, true>(rect, g, s, u, idx, fc, rec, boxes, st);
-    else
-        launch_pre2<SHO, false>(rect, g, s, u, idx, fc, rec, boxes, st);
+static void launch_pre(bool cov, bool rect, const SceneView* s, const Uniforms* u, const uint32_t* idx,
+                       const FrameCounters* fc, float4* rec, uint2* boxes, uint32_t max_n, cudaStream_t st) {
+    constexpr bool CAN_STAGE = SHO > 0;
+    const bool staged = CAN_STAGE && max_n >= PRE_STAGED_MIN;
+    auto run = cov ? (rect ? (staged ? launch_pre3<SHO, true, true, CAN_STAGE> : launch_pre3<SHO, true, true, false>)
+                           : (staged ? launch_pre3<SHO, true, false, CAN_STAGE> : launch_pre3<SHO, true, false, false>))
+                   : (rect ? (staged ? launch_pre3<SHO, false, true, CAN_STAGE> : launch_pre3<SHO, false, true, false>)
+                           : (staged ? launch_pre3<SHO, false, false, CAN_STAGE> : launch_pre3<SHO, false, false, false>));
+    run(s, u, idx, fc, rec, boxes, max_n, st);
 }
 
 void launch_preprocess(int sh_order, bool covariance, bool rect, const SceneView* s, const Uniforms* u,
                        const uint32_t* idx, const FrameCounters* fc, float4* rec, uint2* boxes, uint32_t max_n,
                        cudaStream_t st) {
     if (max_n == 0) return;
-    uint32_t blocks = (max_n + 255) / 256;
-    if (blocks > device_sm_count() * 16u) blocks = device_sm_count() * 16u;
-    const dim3 g(blocks);
-    switch (sh_order) {
-        case 0: launch_pre1<0>(covariance, rect, g, s, u, idx, fc, rec, boxes, st); break;
-        case 1: launch_pre1<1>(covariance, rect, g, s, u, idx, fc, rec, boxes, st); break;
-        case 2: launch_pre1<2>(covariance, rect, g, s, u, idx, fc, rec, boxes, st); break;
-        default: launch_pre1<3>(covariance, rect, g, s, u, idx, fc, rec, boxes, st); break;
-    }
+    auto run = sh_order == 0 ? launch_pre<0> : (sh_order == 1 ? launch_pre<1> : (sh_order == 2 ? launch_pre<2> : launch_pre<3>));
+    run(covariance, rect, s, u, idx, fc, rec, boxes, max_n, st);
 }
 
 // ------------------------------------------------------------------------------------------------

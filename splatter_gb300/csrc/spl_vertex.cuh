@@ -1,6 +1,6 @@
 // The vertex stage of the splat pipeline (Lichtso/splatter src/shaders.wgsl:63-294, 507-573):
-//   vertex_math  -> the forward preprocess kernel (FP32, WGSL operation order, bit-identical to the
-//                   oracle's restatement);
+//   vertex_colour, vertex_shape -> the forward preprocess kernel (FP32, WGSL operation order,
+//                   bit-identical to the oracle's restatement);
 //   vertex_vjp_t -> its vector-Jacobian product for the backward, in reverse mode (float, or double
 //                   for needles and discs), around the forward's own float values.
 // Compiled with -fmad=false; explicit fmaf() only where written.
@@ -135,33 +135,29 @@ __constant__ float c_shc[16] = {
     0.3731763325901154f,   -0.4570457994644658f, 1.445305721320277f,   -0.5900435899266435f,
 };
 
-// sphericalHarmonicsLookup (shaders.wgsl:268-294), one channel; sh coefficients are constants here
-template <int SHO, class S>
-__device__ __forceinline__ S sh_channel(const float* sh, int c, S x, S y, S z, S xx, S yy, S zz) {
-    S col = cst<S>(0.5f);
-    col = col + c_shc[0] * sh[c];
-    if (SHO > 0) {
-        col = col + (c_shc[1] * sh[3 + c]) * y;
-        col = col + (c_shc[2] * sh[6 + c]) * z;
-        col = col + (c_shc[3] * sh[9 + c]) * x;
+// Term K of sphericalHarmonicsLookup (shaders.wgsl:268-294) for coefficient v of one channel; the colour is
+// 0.5 and the terms added in order.
+template <int K>
+__device__ __forceinline__ float sh_term(float v, float x, float y, float z, float xx, float yy, float zz) {
+    const float k = c_shc[K] * v;
+    switch (K) {
+        case 0: return k;
+        case 1: return k * y;
+        case 2: return k * z;
+        case 3: return k * x;
+        case 4: return (k * x) * y;
+        case 5: return (k * y) * z;
+        case 6: return k * ((2.0f * zz - xx) - yy);
+        case 7: return (k * x) * z;
+        case 8: return k * (xx - yy);
+        case 9: return (k * y) * (3.0f * xx - yy);
+        case 10: return ((k * x) * y) * z;
+        case 11: return (k * y) * ((4.0f * zz - xx) - yy);
+        case 12: return (k * z) * ((2.0f * zz - 3.0f * xx) - 3.0f * yy);
+        case 13: return (k * x) * ((4.0f * zz - xx) - yy);
+        case 14: return (k * z) * (xx - yy);
+        default: return (k * x) * (xx - 3.0f * yy);
     }
-    if (SHO > 1) {
-        col = col + ((c_shc[4] * sh[12 + c]) * x) * y;
-        col = col + ((c_shc[5] * sh[15 + c]) * y) * z;
-        col = col + (c_shc[6] * sh[18 + c]) * ((2.0f * zz - xx) - yy);
-        col = col + ((c_shc[7] * sh[21 + c]) * x) * z;
-        col = col + (c_shc[8] * sh[24 + c]) * (xx - yy);
-    }
-    if (SHO > 2) {
-        col = col + ((c_shc[9] * sh[27 + c]) * y) * (3.0f * xx - yy);
-        col = col + (((c_shc[10] * sh[30 + c]) * x) * y) * z;
-        col = col + ((c_shc[11] * sh[33 + c]) * y) * ((4.0f * zz - xx) - yy);
-        col = col + ((c_shc[12] * sh[36 + c]) * z) * ((2.0f * zz - 3.0f * xx) - 3.0f * yy);
-        col = col + ((c_shc[13] * sh[39 + c]) * x) * ((4.0f * zz - xx) - yy);
-        col = col + ((c_shc[14] * sh[42 + c]) * z) * (xx - yy);
-        col = col + ((c_shc[15] * sh[45 + c]) * x) * (xx - 3.0f * yy);
-    }
-    return col;
 }
 
 // The SH basis values B_k(d) with rgb_c = 0.5 + sum_k B_k * sh[3k + c] (the gradient of the colour
@@ -230,29 +226,49 @@ __device__ __forceinline__ void outline_ellipse(const Uniforms& u, float sx, flo
     }
 }
 
-// Everything the vertex stage derives from one splat that the raster uses and that depends on the
-// splat's parameters: the affine pixel -> tc map, the colour, and (for the box) the rect basis.
+// The colour before the fragment falloff (shaders.wgsl:531-532), from a splat's SH row.  FEW_REGISTERS:
+// read four coefficients (three 16-byte pieces) at a time.
+template <int K0, int COEFS, bool FEW_REGISTERS>
+__device__ __forceinline__ void add_sh_terms(const float4* row, float x, float y, float z, float xx, float yy, float zz,
+                                             float (&c)[3]) {
+    if constexpr (K0 < COEFS) {
+        float v[12];
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+            if (4 * p < 3 * (COEFS - K0)) *reinterpret_cast<float4*>(v + 4 * p) = row[3 * K0 / 4 + p];
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) {
+            c[ch] = c[ch] + sh_term<K0>(v[ch], x, y, z, xx, yy, zz);
+            if constexpr (K0 + 1 < COEFS) c[ch] = c[ch] + sh_term<K0 + 1>(v[3 + ch], x, y, z, xx, yy, zz);
+            if constexpr (K0 + 2 < COEFS) c[ch] = c[ch] + sh_term<K0 + 2>(v[6 + ch], x, y, z, xx, yy, zz);
+            if constexpr (K0 + 3 < COEFS) c[ch] = c[ch] + sh_term<K0 + 3>(v[9 + ch], x, y, z, xx, yy, zz);
+        }
+        if constexpr (FEW_REGISTERS) asm volatile("" ::: "memory");  // the next are read after these
+        add_sh_terms<K0 + 4, COEFS, FEW_REGISTERS>(row, x, y, z, xx, yy, zz, c);
+    }
+}
+
+template <int SHO, bool FEW_REGISTERS>
+__device__ __forceinline__ void vertex_colour(const Uniforms& u, float cx, float cy, float cz, const float4* row,
+                                              float (&c)[3]) {
+    const float vx = cx - u.camera[12], vy = cy - u.camera[13], vz = cz - u.camera[14];
+    const float len = sqrtf((vx * vx + vy * vy) + vz * vz);
+    const float x = vx / len, y = vy / len, z = vz / len;
+    c[0] = c[1] = c[2] = 0.5f;
+    add_sh_terms<0, (SHO + 1) * (SHO + 1), FEW_REGISTERS>(row, x, y, z, x * x, y * y, z * z, c);
+}
+
+// The shape of a splat on the screen: the affine pixel -> tc map and (for the box) the rect basis.
 template <class S>
-struct VertexOut {
+struct VertexShape {
     S A00, A01, B0, A10, A11, B1;  // tc = (A00 X + A01 Y + B0, A10 X + A11 Y + B1)
-    S cr, cg, cb;                  // colour before the fragment falloff
     S Xx, Xy, Yx, Yy, t0, t1;      // rect basis (shaders.wgsl:543-547)
     float bx, by;                  // AA-square offsets
 };
 
-template <int SHO, bool COV, class S>
-__device__ __forceinline__ void vertex_math(const Uniforms& u, S cx, S cy, S cz, S q0, S q1, S q2, S q3, S scx, S scy,
-                                            S scz, const float* sh, VertexOut<S>& o) {
-    // colour (shaders.wgsl:531-532)
-    {
-        const S vx = cx - u.camera[12], vy = cy - u.camera[13], vz = cz - u.camera[14];
-        const S len = sqrt_((vx * vx + vy * vy) + vz * vz);
-        const S dx = vx / len, dy = vy / len, dz = vz / len;
-        const S dxx = dx * dx, dyy = dy * dy, dzz = dz * dz;
-        o.cr = sh_channel<SHO>(sh, 0, dx, dy, dz, dxx, dyy, dzz);
-        o.cg = sh_channel<SHO>(sh, 1, dx, dy, dz, dxx, dyy, dzz);
-        o.cb = sh_channel<SHO>(sh, 2, dx, dy, dz, dxx, dyy, dzz);
-    }
+template <bool COV, class S>
+__device__ __forceinline__ void vertex_shape(const Uniforms& u, S cx, S cy, S cz, S q0, S q1, S q2, S q3, S scx, S scy,
+                                             S scz, VertexShape<S>& o) {
     // conic + decomposition (shaders.wgsl:533-542)
     const S sx = scx * u.splat_scale, sy = scy * u.splat_scale, sz = scz * u.splat_scale;
     S t0, t1, rj, rk, ax0, ax1;
@@ -300,7 +316,7 @@ __device__ __forceinline__ T m3(const M3T<T>& X, int r, int c) {
 }
 
 // Gradient of one SH colour channel with respect to the unit view direction (x, y, z): the derivative
-// of sh_channel's polynomial term by term (xx = x^2 ...), accumulated with weight gc into gd.
+// of sh_term's polynomials term by term (xx = x^2 ...), accumulated with weight gc into gd.
 template <int SHO, class T>
 __device__ __forceinline__ void sh_channel_grad(const float* sh, int c, T gc, T x, T y, T z, T xx, T yy, T zz, T* gd) {
     T gx = 0.0f, gy = 0.0f, gz = 0.0f;
