@@ -269,7 +269,8 @@ int spl_renderer_create(const spl_config* cfg, spl_renderer** out) {
     TRY(dalloc(&r->epoch, 1));
     TRY(dalloc(&r->d_u, 1));
     TRY(dalloc(&r->d_sv, 1));
-    TRY(dalloc(&r->coop_cnt, 256 * (((size_t)sort_coop_grid() + 3) & ~(size_t)3) + 256));
+    TRY(dalloc(&r->coop_table, 2 * sort_coop_table_words()));
+    (void)sort_coop_grid();  // its one-time occupancy query, outside any stream capture
 #undef TRY
     cudaError_t e = cudaSuccess;
     // status words start at epoch 0, which no frame uses
@@ -278,7 +279,7 @@ int spl_renderer_create(const spl_config* cfg, spl_renderer** out) {
     if (e == cudaSuccess) e = cudaMemset(r->fc, 0, sizeof(FrameCounters));
     if (e == cudaSuccess) e = cudaMemset(r->fc_sort, 0, sizeof(FrameCounters));
     if (e == cudaSuccess)
-        e = cudaMemset(r->coop_cnt, 0, (256 * (((size_t)sort_coop_grid() + 3) & ~(size_t)3) + 256) * 4);
+        e = cudaMemset(r->coop_table, 0, 2 * sort_coop_table_words() * 8);
     if (e == cudaSuccess) e = cudaMemset(r->epoch, 0, 4);
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&r->host_fc), sizeof(FrameCounters));
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -340,7 +341,7 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
         // four stable 8-bit passes a -> b -> a -> b -> a; pass 0 takes the compaction slot as the value
         if (coop) {
             CU(launch_sort_coop(r->keys_a, r->keys_b, r->vals_a, r->vals_b, true, &r->fc->visible, N, 4, 0,
-                                r->coop_cnt, r->fc->barrier, sl, &r->fc->err, st));
+                                r->coop_table, r->epoch, r->fc->barrier, sl, &r->fc->err, st));
         } else {
             // digit histograms from the cull kernel; one launch per pass
             uint32_t *src_k = r->keys_a, *dst_k = r->keys_b, *dst_v = r->vals_b;
@@ -369,7 +370,7 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
     const int passes = tiles <= 256 ? 1 : (tiles <= 65536 ? 2 : 3);
     if (coop) {
         CU(launch_sort_coop(r->pk_a, r->pk_b, r->pv_a, r->pv_b, false, &r->fc->pairs, (uint32_t)r->pair_cap, passes,
-                            0, r->coop_cnt, r->fc->barrier + 1, sl, &r->fc->err, st));
+                            0, r->coop_table + sort_coop_table_words(), r->epoch, r->fc->barrier + 1, sl, &r->fc->err, st));
     } else {
         // tile-id histograms from the binning kernel
         uint32_t *ak = r->pk_a, *av = r->pv_a, *bk = r->pk_b, *bv = r->pv_b;
@@ -627,7 +628,7 @@ int spl_sort_pairs(spl_renderer* r, const uint32_t* keys_in, const uint32_t* val
     CU(cudaMemcpyAsync(r->keys_a, keys_in, count * 4, cudaMemcpyDeviceToDevice, st));
     CU(cudaMemcpyAsync(r->vals_a, values_in, count * 4, cudaMemcpyDeviceToDevice, st));
     CU(launch_sort_coop(r->keys_a, r->keys_b, r->vals_a, r->vals_b, false, &r->fc_sort->visible, (uint32_t)count,
-                        passes, 0, r->coop_cnt, r->fc_sort->barrier, r->spin_limit, &r->fc_sort->err, st));
+                        passes, 0, r->coop_table, r->epoch, r->fc_sort->barrier, r->spin_limit, &r->fc_sort->err, st));
     const uint32_t* kr = (passes & 1) ? r->keys_b : r->keys_a;
     const uint32_t* vr = (passes & 1) ? r->vals_b : r->vals_a;
     CU(cudaMemcpyAsync(keys_out, kr, count * 4, cudaMemcpyDeviceToDevice, st));

@@ -83,7 +83,7 @@ struct spl_renderer {
     uint32_t *pk_a = nullptr, *pk_b = nullptr, *pv_a = nullptr, *pv_b = nullptr;
     FrameCounters* fc = nullptr;
     FrameCounters* fc_sort = nullptr;  // counters of spl_sort_pairs
-    uint32_t* coop_cnt = nullptr;      // [256][grid, padded to 4] digit counts + [256] totals (cooperative sort)
+    uint64_t* coop_table = nullptr;    // count words of the cooperative depth sort, then of the pair sort
     uint32_t* epoch = nullptr;
     Uniforms* d_u = nullptr;           // the frame's uniform block in device memory (k_frame_begin writes it)
     SceneView* d_sv = nullptr;         // the frame's scene view in device memory (k_frame_begin writes it)
@@ -121,7 +121,7 @@ struct spl_renderer {
         dfree(keys_a); dfree(keys_b); dfree(vals_a); dfree(vals_b); dfree(idx); dfree(rec); dfree(boxes); dfree(grad_rec); dfree(grad_deferred);
         dfree(st_cull); dfree(st_bin);
         dfree(pk_a); dfree(pk_b); dfree(pv_a); dfree(pv_b);
-        dfree(fc); dfree(fc_sort); dfree(coop_cnt); dfree(epoch); dfree(ranges); dfree(tile_order); dfree(d_u); dfree(d_sv);
+        dfree(fc); dfree(fc_sort); dfree(coop_table); dfree(epoch); dfree(ranges); dfree(tile_order); dfree(d_u); dfree(d_sv);
         dfree(st_sort); dfree(st_pairs);
         if (host_fc) cudaFreeHost(host_fc);
         host_fc = nullptr;

@@ -112,11 +112,14 @@ void launch_soa_to_splats60(const SceneView& s, uint32_t start, uint32_t count, 
 void launch_gather_entries(const uint32_t* keys, const uint32_t* slots, const uint32_t* idx, const FrameCounters* fc,
                            int mode, uint32_t* keys_out, uint32_t* idx_out, uint32_t cap, cudaStream_t st);
 // All passes of a stable LSD radix sort in one cooperative launch (k_sort_coop.cu).  Pass p reads
-// buffers (p even: 0, odd: 1) and writes the other; cnt holds 256 x sort_coop_grid() words; *bar (the
-// grid barrier's arrival count) must be zero when the launch starts.
+// buffers (p even: 0, odd: 1) and writes the other.  table: sort_coop_table_words() words of its own for each
+// sort of a frame, zero at first and never cleared (the words carry *epoch_word, never 0 and another one at
+// each launch); *bar (the grid barrier's arrival count) must be zero when the launch starts.
 cudaError_t launch_sort_coop(uint32_t* keys0, uint32_t* keys1, uint32_t* vals0, uint32_t* vals1, bool iota_first,
-                             const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0, uint32_t* cnt,
-                             uint32_t* bar, uint32_t spin_limit, uint32_t* err, cudaStream_t st);
+                             const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0, uint64_t* table,
+                             const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit, uint32_t* err,
+                             cudaStream_t st);
+size_t sort_coop_table_words();
 int sort_coop_grid();
 // The loader's activations of raw parameters and their backward (k_activate.cu).
 void launch_activate(uint32_t n, const float* means, const float* quats, const float* logs, const float* logits,
