@@ -362,9 +362,8 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
         order = r->vals_a;  // keys in keys_a
     }
     r->mark(3, st);
-    CU(cudaMemsetAsync(r->ranges, 0, tiles * sizeof(uint2), st));
     launch_bin(mode, !coop, order, r->boxes, r->fc, r->epoch, r->st_bin, r->pk_a, r->pv_a, (uint32_t)r->pair_cap,
-               (int)tiles_x, N, sl, st);
+               (int)tiles_x, r->ranges, (uint32_t)tiles, N, sl, st);
     r->mark(4, st);
     // stable sort of the pairs by tile id keeps each tile's list in depth order
     const int passes = tiles <= 256 ? 1 : (tiles <= 65536 ? 2 : 3);
@@ -514,9 +513,9 @@ int spl_renderer_launches_per_frame(const spl_renderer* r, uint32_t width, uint3
     const bool coop = r->sort_mode == SPL_SORT_COOPERATIVE;
     const int depth_sort = r->cfg.depth_sorting == DS_NONE ? 0 : (coop ? 1 : 4);
     // frame_begin, cull, preprocess, depth sort (one cooperative launch or 4 onesweep passes),
-    // ranges memset, bin, pair sort (one cooperative launch or one launch per pass), ranges, tile
+    // bin, pair sort (one cooperative launch or one launch per pass), ranges, tile
     // order, raster
-    return 1 + 1 + 1 + depth_sort + 1 + 1 + (coop ? 1 : pair_passes) + 1 + (r->order_tiles ? 1 : 0) + 1;
+    return 1 + 1 + 1 + depth_sort + 1 + (coop ? 1 : pair_passes) + 1 + (r->order_tiles ? 1 : 0) + 1;
 }
 
 static int render_backward(spl_renderer* r, const spl_scene* scene, const float* image_device,

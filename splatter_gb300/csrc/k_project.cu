@@ -37,6 +37,8 @@ __global__ void k_counters_begin(FrameCounters* fc, uint32_t* epoch_word) { coun
 // this one node) published to device memory for the kernels that follow.
 __global__ void k_frame_begin(FrameCounters* fc, uint32_t* epoch_word, Uniforms u, Uniforms* d_u, SceneView sv,
                               SceneView* d_sv) {
+    start_next();
+    frame_step();
     if (threadIdx.x < sizeof(Uniforms) / 4)
         reinterpret_cast<uint32_t*>(d_u)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&u)[threadIdx.x];
     if (threadIdx.x < sizeof(SceneView) / 4)
@@ -83,6 +85,7 @@ __global__ void __launch_bounds__(256, 3) k_cull_key(const SceneView* __restrict
     const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
     if (HIST)
         for (uint32_t i = tid; i < 1024u; i += 256u) s_hist[i] = 0u;
+    frame_step(d_sv, d_u, epoch_word);
     stage_frame(d_u, s_u, d_sv, s_sv);
     if (tid == 0) {
         s_tile = atomicAdd(&fc->tile_counter[0], 1u);
@@ -200,7 +203,7 @@ void launch_cull_key(int mode, bool hist, uint32_t grid_n, const SceneView* d_sv
     const uint32_t grid = (grid_n + CULL_TILE - 1) / CULL_TILE;
     auto k = mode == DS_CPU ? (hist ? k_cull_key<DS_CPU, true> : k_cull_key<DS_CPU, false>)
                             : (hist ? k_cull_key<DS_GPU, true> : k_cull_key<DS_GPU, false>);
-    k<<<grid, 256, 0, st>>>(d_sv, u, fc, epoch_word, status, keys_out, idx_out, spin_limit);
+    launch_after(k, grid, 256, st, d_sv, u, fc, epoch_word, status, keys_out, idx_out, spin_limit);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -239,6 +242,7 @@ __global__ void __launch_bounds__(PreShape<SHO, STAGED>::WARPS * 32, PreShape<SH
     __shared__ float4 s_sh[PreShape<SHO, STAGED>::WARPS][STAGED ? 32 * STRIDE : 1];
     __shared__ Uniforms s_u;
     __shared__ SceneView s_sv;
+    frame_step(d_sv, d_u, idx, fc);
     stage_frame(d_u, s_u, d_sv, s_sv);
     __syncthreads();
     const Uniforms& u = s_u;
@@ -339,7 +343,7 @@ static void launch_pre3(const SceneView* s, const Uniforms* u, const uint32_t* i
     constexpr uint32_t threads = PreShape<SHO, STAGED>::WARPS * 32;
     // grid stride beyond 4096 threads per SM
     const uint32_t blocks = (max_n + threads - 1) / threads, cap = device_sm_count() * (4096u / threads);
-    k_preprocess<SHO, COV, RECT, STAGED><<<blocks < cap ? blocks : cap, threads, 0, st>>>(s, u, idx, fc, rec, boxes);
+    launch_after(k_preprocess<SHO, COV, RECT, STAGED>, blocks < cap ? blocks : cap, threads, st, s, u, idx, fc, rec, boxes);
 }
 template <int SHO>
 static void launch_pre(bool cov, bool rect, const SceneView* s, const Uniforms* u, const uint32_t* idx,

@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(256) k_bin(const uint32_t* __restrict__ order,
                                              FrameCounters* fc, int mode, const uint32_t* __restrict__ epoch_word,
                                              uint64_t* status, uint32_t* __restrict__ pair_keys,
                                              uint32_t* __restrict__ pair_vals, uint32_t pair_cap, int tiles_x,
-                                             uint32_t spin_limit) {
+                                             uint2* __restrict__ ranges, uint32_t tiles, uint32_t spin_limit) {
     __shared__ uint32_t s_off[BIN_TILE];  // exclusive pair offsets of the tile's entries
     __shared__ uint32_t s_slot[BIN_TILE];
     __shared__ uint32_t s_box[BIN_TILE];  // tx0 | ty0 << 16
@@ -35,6 +35,9 @@ __global__ void __launch_bounds__(256) k_bin(const uint32_t* __restrict__ order,
     __shared__ uint32_t s_scan[8];
     __shared__ uint32_t s_tile, s_epoch, s_base, s_draw;
     const uint32_t tid = threadIdx.x;
+    frame_step(order, boxes, epoch_word);
+    // every tile's range starts empty
+    for (uint32_t i = blockIdx.x * 256u + tid; i < tiles; i += gridDim.x * 256u) ranges[i] = make_uint2(0u, 0u);
     if (tid == 0) {
         s_tile = atomicAdd(&fc->tile_counter[8], 1u);
         s_epoch = *epoch_word;
@@ -188,16 +191,18 @@ __global__ void __launch_bounds__(256) k_bin(const uint32_t* __restrict__ order,
 
 void launch_bin(int mode, bool hist, const uint32_t* order, const uint2* boxes, FrameCounters* fc,
                 const uint32_t* epoch_word, uint64_t* status, uint32_t* pair_keys, uint32_t* pair_vals,
-                uint32_t pair_cap, int tiles_x, uint32_t max_n, uint32_t spin_limit, cudaStream_t st) {
+                uint32_t pair_cap, int tiles_x, uint2* ranges, uint32_t tiles, uint32_t max_n, uint32_t spin_limit,
+                cudaStream_t st) {
     const uint32_t grid = max_n == 0 ? 1u : (max_n + BIN_TILE - 1) / BIN_TILE;
     auto k = order ? (hist ? k_bin<true, true> : k_bin<true, false>) : (hist ? k_bin<false, true> : k_bin<false, false>);
-    k<<<grid, 256, 0, st>>>(order, boxes, fc, mode, epoch_word, status, pair_keys, pair_vals, pair_cap, tiles_x,
-                            spin_limit);
+    launch_after(k, grid, 256, st, order, boxes, fc, mode, epoch_word, status, pair_keys, pair_vals, pair_cap, tiles_x,
+                 ranges, tiles, spin_limit);
 }
 
 // ------------------------------------------------------------------------------------------------
 __global__ void k_tile_ranges(const uint32_t* __restrict__ keys, const FrameCounters* __restrict__ fc,
                               uint32_t pair_cap, uint2* ranges) {
+    frame_step(keys, fc);
     const uint32_t P = min(fc->pairs, pair_cap);
     // four keys per thread (one 16-byte load; the neighbours across the group edges loaded singly)
     const uint32_t groups = (P + 3u) / 4u;
@@ -234,7 +239,7 @@ void launch_tile_ranges(const uint32_t* pair_keys, const FrameCounters* fc, uint
     if (pair_cap == 0) return;
     uint32_t grid = (pair_cap + 255) / 256;
     if (grid > device_sm_count() * 8u) grid = device_sm_count() * 8u;
-    k_tile_ranges<<<grid, 256, 0, st>>>(pair_keys, fc, pair_cap, ranges);
+    launch_after(k_tile_ranges, grid, 256, st, pair_keys, fc, pair_cap, ranges);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -262,6 +267,8 @@ __global__ void __launch_bounds__(1024) k_tile_order(const uint2* __restrict__ r
     __shared__ uint8_t bkt[ORDER_SMEM_TILES];
     const uint32_t lane = threadIdx.x & 31u;
     if (threadIdx.x < ORDER_BUCKETS) cnt[threadIdx.x] = 0u;
+    start_next();
+    frame_step(ranges);
     __syncthreads();
     // histogram; lanes of a warp with the same bucket add once (most tiles share a few buckets)
 #pragma unroll 4
@@ -419,6 +426,7 @@ __global__ void __launch_bounds__(256, 6) k_raster(const uint2* __restrict__ ran
     // [strip][record]: lane masks of the batch's records; then [strip][word * 32 + lane]: the pixels' lists
     __shared__ uint32_t s_pm[8][RASTER_BATCH];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+    frame_step(ranges, tile_order, pair_vals, rec);
     const int tile = tile_order ? (int)__ldg(tile_order + blockIdx.x) : (int)blockIdx.x;
     const int tx = tile % tiles_x, ty = tile / tiles_x;
     const int wx0 = tx * TILE_PIXELS;
@@ -596,9 +604,9 @@ void launch_raster(bool rect, int blend, const uint2* ranges, uint32_t* tile_ord
     if (grid == 0) return;
     const float psx = (2.0f * u.view_size[0]) / (float)W;
     const float psy = -((2.0f * u.view_size[1]) / (float)H);
-    if (tile_order) k_tile_order<<<1, 1024, 0, st>>>(ranges, (uint32_t)grid, tile_order);
-    pick_raster(rect, blend, u.margin)<<<grid, 256, 0, st>>>(ranges, tile_order, pair_vals, rec, W, H, tiles_x, u.margin,
-                                                             psx, psy, out);
+    if (tile_order) launch_after(k_tile_order, 1, 1024, st, ranges, (uint32_t)grid, tile_order);
+    launch_after(pick_raster(rect, blend, u.margin), (uint32_t)grid, 256, st, ranges, tile_order, pair_vals, rec, W, H,
+                 tiles_x, u.margin, psx, psy, out);
 }
 
 }  // namespace spl

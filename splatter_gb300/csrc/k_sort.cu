@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(OS_THREADS, 3)
     __shared__ uint32_t s_scan[8];
     __shared__ uint32_t s_tile;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+    frame_step(keys_in, vals_in, n_ptr, hist256, epoch_word);
     const uint32_t n = min(*n_ptr, n_cap);
     const uint32_t ntiles = (n + SORT_TILE - 1) / SORT_TILE;
     const uint32_t epoch = *epoch_word;
@@ -175,11 +176,11 @@ void launch_onesweep(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t*
     uint32_t grid = (uint32_t)(shape.num_sms * shape.blocks_per_sm);
     if (grid > tiles) grid = tiles;
     if (vals_in == nullptr)
-        k_onesweep<true><<<grid, OS_THREADS, 0, st>>>(keys_in, vals_in, keys_out, vals_out, n_ptr, n_cap, hist256,
-                                                       status, tile_counter, epoch_word, shift, spin_limit, err);
+        launch_after(k_onesweep<true>, grid, OS_THREADS, st, keys_in, vals_in, keys_out, vals_out, n_ptr, n_cap, hist256,
+                     status, tile_counter, epoch_word, shift, spin_limit, err);
     else
-        k_onesweep<false><<<grid, OS_THREADS, 0, st>>>(keys_in, vals_in, keys_out, vals_out, n_ptr, n_cap, hist256,
-                                                        status, tile_counter, epoch_word, shift, spin_limit, err);
+        launch_after(k_onesweep<false>, grid, OS_THREADS, st, keys_in, vals_in, keys_out, vals_out, n_ptr, n_cap, hist256,
+                     status, tile_counter, epoch_word, shift, spin_limit, err);
 }
 
 // Digit histograms of all four 8-bit places of `n` keys (the upsweep the standalone sort needs;

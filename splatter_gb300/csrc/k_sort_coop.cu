@@ -444,6 +444,7 @@ __global__ void __launch_bounds__(CS_THREADS, 2)
     CoopSmem& sm = *reinterpret_cast<CoopSmem*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
     const uint32_t c = blockIdx.x;
+    frame_step(n_ptr, epoch_word);
     const uint32_t n = min(*n_ptr, n_cap);
     // Contiguous segments, 256-aligned: up to one sub-tile of keys is one CTA's work, more are spread over
     // the grid in segments of at least CS_MIN_SEG.  The live count is read on the device (a captured graph

@@ -15,6 +15,40 @@ namespace spl {
 constexpr uint32_t FULL_MASK = 0xFFFFFFFFu;
 
 // ------------------------------------------------------------------------------------------------
+// A frame's kernels are launched with programmatic dependence (launch_after): a kernel's blocks may start when
+// every block of the kernel before it has ended or called start_next, instead of after a full launch latency.
+// Every kernel calls frame_step before it touches memory: it waits until the kernel before has ended and its
+// writes are visible (at once, where a kernel is launched plainly), so a kernel sees all kernels before it
+// complete.  The pointers that it reads through the read-only path are given to frame_step: the compiler
+// takes what such loads read for unchanging and might read it before the wait otherwise.
+// Frames of 2k splats 44.6 -> 38.3 us, of 100k 101.4 -> 99.4 us, of 1M 188.3 -> 187.1 us, of 6M the same.
+// start_next is called by the kernels of one block only (frame start, tile order: thumbnails and 1M splats gain
+// 0.4 and 1.3 us); called by all, the next kernel's waiting blocks take room from the last wave (100k splats
+// 105.5 us, 6M +10 us), and the cooperative sorts stay plain dependents for the same reason.
+// ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P>
+__device__ __forceinline__ void frame_step(P&... read_only) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    (([&] { asm volatile("" : "+l"(read_only)::"memory"); }()), ...);
+}
+
+template <class... Params, class... Args>
+inline cudaError_t launch_after(void (*kernel)(Params...), uint32_t grid, uint32_t threads, cudaStream_t st, Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+// ------------------------------------------------------------------------------------------------
 // Decoupled look-back status words: [epoch:32 | INC:1 | AGG:1 | value:30].  A word is only valid
 // when its epoch equals the frame's epoch, so status arrays never need clearing between frames.
 // ------------------------------------------------------------------------------------------------

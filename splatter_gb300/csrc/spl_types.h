@@ -94,10 +94,12 @@ void launch_onesweep(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t*
                      const uint32_t* n_ptr, uint32_t n_cap, const uint32_t* hist256, uint64_t* status,
                      uint32_t* tile_counter, const uint32_t* epoch_word, int shift, uint32_t spin_limit,
                      uint32_t* err, cudaStream_t st);
-// hist: also build the digit histograms of the pairs' tile ids (the onesweep passes need them).
+// hist: also build the digit histograms of the pairs' tile ids (the onesweep passes need them).  Empties the
+// `tiles` entries of ranges.
 void launch_bin(int mode, bool hist, const uint32_t* order, const uint2* boxes, FrameCounters* fc,
                 const uint32_t* epoch_word, uint64_t* status, uint32_t* pair_keys, uint32_t* pair_vals,
-                uint32_t pair_cap, int tiles_x, uint32_t max_n, uint32_t spin_limit, cudaStream_t st);
+                uint32_t pair_cap, int tiles_x, uint2* ranges, uint32_t tiles, uint32_t max_n, uint32_t spin_limit,
+                cudaStream_t st);
 void launch_tile_ranges(const uint32_t* pair_keys, const FrameCounters* fc, uint32_t pair_cap, uint2* ranges,
                         cudaStream_t st);
 // Orders the tiles most pairs first (tile_order, one entry per tile), then rasterises them in that order;
