@@ -12,7 +12,7 @@
 //     dL/ds_c  = dL/dC_c * T_i
 //     dL/dsa   = -(dL/dC . S + dL/dT * T_final) / (1 - sa)
 // and the chain through sat(), the falloff and tc = A (X, Y) + B gives per-splat gradients of the
-// record (A00, A01, B0, A10, A11, B1, a, r, g, b), reduced over each 8-lane pixel group before one
+// record (A00, A01, B0, A10, A11, B1, a, r, g, b), reduced over each 2x2-pixel group before one
 // set of global float atomics per (splat, group).  A is accumulated against pixel offsets from the
 // centre of the splat's pixel box and B at that centre (well conditioned; see vertex_vjp_t).
 //
@@ -21,6 +21,7 @@
 // sweep of adjoints back through the same formulas, in float; needles and discs (needs_double_sweep)
 // are left to k_preprocess_backward_double, which sweeps them in double.  SH coefficient gradients
 // are the basis values times the colour gradients.
+#include "spl_raster.cuh"
 #include "spl_vertex.cuh"
 
 namespace spl {
@@ -33,36 +34,37 @@ __global__ void k_zero_grad_rec(float* grad_rec, const FrameCounters* fc, uint32
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) grad_rec[i] = 0.0f;
 }
 
-// Sums 10 values over the 8 lanes of a lane group (lane index li = lane & 7) in three exchange steps
-// that halve the values each lane carries (5 + 3 + 2 shuffles instead of 3 per value): afterwards lane
-// li holds the group sum of value k0 in v0 and, for li = 0 and 4, of value k0 + 1 in v1.
-//   li: 0 -> 0, 1   1 -> 2   2 -> 3   3 -> 4   4 -> 5, 6   5 -> 7   6 -> 8   7 -> 9
-__device__ __forceinline__ uint32_t reduce10_over8(const float* g, uint32_t li, float& v0, float& v1) {
-    const bool h4 = (li & 4u) != 0u, h2 = (li & 2u) != 0u, h1 = (li & 1u) != 0u;
-    float a[5], b[3];
+// Sums 10 values over the 4 lanes of a lane group in two exchange steps that halve the values each lane carries:
+// lane li = 2 h2 + h1 gets the sums of values k0 = 5 h2 + 3 h1 on, three of them (h1 = 0) or two.
+__device__ __forceinline__ uint32_t reduce10_over4(const float* g, uint32_t li, float (&v)[3]) {
+    const bool h2 = (li & 2u) != 0u, h1 = (li & 1u) != 0u;
+    float a[5];
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {  // keep values 5..9 (h4) or 0..4
-        const float send = h4 ? g[i] : g[i + 5], keep = h4 ? g[i + 5] : g[i];
-        a[i] = keep + __shfl_xor_sync(FULL_MASK, send, 4);
+    for (int i = 0; i < 5; ++i) {  // keep values 5..9 (h2) or 0..4
+        const float send = h2 ? g[i] : g[i + 5], keep = h2 ? g[i + 5] : g[i];
+        a[i] = keep + __shfl_xor_sync(FULL_MASK, send, 2);
     }
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {  // keep a[3..4] (h2) or a[0..2]
+    for (int i = 0; i < 3; ++i) {  // keep a[3..4] (h1) or a[0..2]
         const float hi = i < 2 ? a[i + 3] : 0.0f;
-        const float send = h2 ? a[i] : hi, keep = h2 ? hi : a[i];
-        b[i] = keep + __shfl_xor_sync(FULL_MASK, send, 2);
+        const float send = h1 ? a[i] : hi, keep = h1 ? hi : a[i];
+        v[i] = keep + __shfl_xor_sync(FULL_MASK, send, 1);
     }
-    // h2 lanes carry two values (b0, b1): keep b1 (h1) or b0; the others three: keep b2 (h1) or b0, b1
-    const float send0 = h1 ? b[0] : (h2 ? b[1] : b[2]);
-    const float keep0 = h1 ? (h2 ? b[1] : b[2]) : b[0];
-    const float send1 = (h1 && !h2) ? b[1] : 0.0f;
-    const float keep1 = (!h1 && !h2) ? b[1] : 0.0f;
-    v0 = keep0 + __shfl_xor_sync(FULL_MASK, send0, 1);
-    v1 = keep1 + __shfl_xor_sync(FULL_MASK, send1, 1);
-    return (h4 ? 5u : 0u) + (h2 ? (h1 ? 4u : 3u) : (h1 ? 2u : 0u));
+    return (h2 ? 5u : 0u) + (h1 ? 3u : 0u);
 }
 
-template <bool RECT>
-__global__ void __launch_bounds__(256) k_raster_backward(const uint2* __restrict__ ranges,
+// One CTA per tile, its warps as in k_raster (strips of two rows), a warp's lanes in eight groups of 2x2 pixels.
+// A group walks its own list of the batch's records, those whose row masks (mask_rows) touch one of its pixels,
+// all four lanes on the same record, so that the record's ten gradients are summed over the group before they
+// are added to grad_rec.  The lists are record indices in shared memory: eight ballots per 32 records give every
+// (record, group) its place, and the walk has no list bookkeeping but a counter.
+// Bound by instruction issue (70% of the slots at 32 warps per SM, DRAM 7%): what counts is the number of walk
+// iterations, i.e. how well the lists fit, and what one costs.  Per view of 1M splats at 1024x1024, 8 views:
+// groups of 4x2 pixels listed by their boxes and walked in lockstep over 32 records 167 us; lists from the row
+// masks, walked over the whole batch, 134 us; groups of 2x2 pixels (fewer idle lanes, two exchange steps instead
+// of three, more atomics) 116 us; lists as record indices instead of bit words 111 us.
+template <bool RECT, bool FAR>
+__global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restrict__ ranges,
                                                          const uint32_t* __restrict__ tile_order,
                                                          const uint32_t* __restrict__ pair_vals,
                                                          const float4* __restrict__ rec, int W, int H, int tiles_x,
@@ -70,18 +72,21 @@ __global__ void __launch_bounds__(256) k_raster_backward(const uint2* __restrict
                                                          const float4* __restrict__ image,
                                                          const float4* __restrict__ grad_image,
                                                          float* __restrict__ grad_rec) {
-    __shared__ float4 s_q0[256], s_q1[256], s_q2[256];
-    __shared__ float4 s_q3[RECT ? 1 : 256];
-    __shared__ uint32_t s_slot[256];
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
-    const uint32_t grp = lane >> 3, li = lane & 7u;
+    // (A00, A10, A01, A11) (B0, B1, alpha, r) (g, b, centre of the pixel box)
+    __shared__ float4 s_a[RASTER_BATCH], s_b[RASTER_BATCH], s_c[RASTER_BATCH];
+    __shared__ float4 s_q3[RECT ? 1 : RASTER_BATCH];
+    __shared__ uint32_t s_row[RASTER_BATCH], s_pm[8][RASTER_BATCH];  // the record's row of grad_rec; its row masks
+    __shared__ uint8_t s_list[8][8][RASTER_BATCH];                   // [warp][group]
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5, lt = lanemask_lt();
+    const uint32_t grp = lane >> 2, li = lane & 3u;
     // the forward's most-pairs-first order of this frame's tiles, when it made one
     const int tile = tile_order ? (int)__ldg(tile_order + blockIdx.x) : (int)blockIdx.x;
     const int tx = tile % tiles_x, ty = tile / tiles_x;
-    const int bx0 = tx * TILE_PIXELS + 4 * (int)grp;
-    const int by0 = ty * TILE_PIXELS + 2 * (int)w;
-    const int px = bx0 + (int)(li & 3u), py = by0 + (int)(li >> 2);
+    const int wx0 = tx * TILE_PIXELS, ty0 = ty * TILE_PIXELS;
+    const uint32_t col = 2u * grp + (li & 1u), row = li >> 1;
+    const int px = wx0 + (int)col, py = ty0 + 2 * (int)w + (int)row;
     const float X = (float)px + 0.5f, Y = (float)py + 0.5f;
+    const uint32_t my_pixel = 1u << (16u * row + col);  // in a strip's row mask
     const uint2 rg = ranges[tile];
     const bool inside = px < W && py < H;
     float Cf[3] = {0.0f, 0.0f, 0.0f}, gC[3] = {0.0f, 0.0f, 0.0f}, Tf = 1.0f, gT = 0.0f;
@@ -95,127 +100,127 @@ __global__ void __launch_bounds__(256) k_raster_backward(const uint2* __restrict
     bool done = !inside;
     float T = 1.0f, Ca[3] = {0.0f, 0.0f, 0.0f};
     const float alpha_min = 1.0f / 255.0f;
-    const int wx0 = tx * TILE_PIXELS;
-    for (uint32_t b = rg.x; b < rg.y; b += 256) {
-        __syncthreads();
+    for (uint32_t b = rg.x; b < rg.y; b += RASTER_BATCH) {
         const uint32_t i = b + tid;
+#pragma unroll
+        for (int sw = 0; sw < 8; ++sw) s_pm[sw][tid] = 0u;
         if (i < rg.y) {
-            const uint32_t slot = __ldg(pair_vals + i);
-            s_slot[tid] = slot;
-            const float4* r = rec + (size_t)slot * 4;
-            s_q0[tid] = __ldg(r + 0);
-            s_q1[tid] = __ldg(r + 1);
-            s_q2[tid] = __ldg(r + 2);
+            const uint32_t rs = __ldg(pair_vals + i);
+            const float4* r = rec + (size_t)rs * 4;
+            const float4 r0 = __ldg(r + 0), r1 = __ldg(r + 1), r2 = __ldg(r + 2);
+            const uint32_t lo = __float_as_uint(r1.w), hi = __float_as_uint(r2.w);
+            s_row[tid] = rs;
+            s_a[tid] = make_float4(r0.x, r0.w, r0.y, r1.x);
+            s_b[tid] = make_float4(r0.z, r1.y, r1.z, r2.x);
+            s_c[tid] = make_float4(r2.y, r2.z, 0.5f * (float)((lo & 0xFFFFu) + (hi & 0xFFFFu) + 1u),
+                                   0.5f * (float)((lo >> 16) + (hi >> 16) + 1u));
             if (!RECT) s_q3[tid] = __ldg(r + 3);
+            mask_rows<RECT>(s_pm, tid, r0, r1, r2, wx0, ty0, margin);
         }
         __syncthreads();
-        const uint32_t cnt = min(256u, rg.y - b);
         if (__any_sync(FULL_MASK, !done)) {
-            for (uint32_t j0 = 0; j0 < cnt; j0 += 32) {
-                uint32_t m0, m1, m2, m3;
-                {
-                    const uint32_t jl = j0 + lane;
-                    int x0 = 1, x1 = 0, y0 = 1, y1 = 0;
-                    if (jl < cnt) {
-                        const uint32_t lo = __float_as_uint(s_q1[jl].w), hi = __float_as_uint(s_q2[jl].w);
-                        x0 = (int)(lo & 0xFFFFu);
-                        y0 = (int)(lo >> 16);
-                        x1 = (int)(hi & 0xFFFFu);
-                        y1 = (int)(hi >> 16);
+            uint32_t count = 0u, longest = 0u;  // entries of this lane's group's list, and of the warp's longest
+            {
+                uint32_t n[8] = {};
+#pragma unroll 1
+                for (uint32_t c = 0; c < RASTER_BATCH; c += 32u) {
+                    const uint32_t m = s_pm[w][c + lane];
+                    if (!__any_sync(FULL_MASK, m != 0u)) continue;
+#pragma unroll
+                    for (uint32_t q = 0; q < 8u; ++q) {
+                        const bool hit = (m & (0x00030003u << (2u * q))) != 0u;
+                        const uint32_t hits = __ballot_sync(FULL_MASK, hit);
+                        if (hit) s_list[w][q][n[q] + __popc(hits & lt)] = (uint8_t)(c + lane);
+                        n[q] += __popc(hits);
                     }
-                    const bool rows = !(y1 < by0 || y0 > by0 + 1) && x0 <= x1;
-                    m0 = __ballot_sync(FULL_MASK, rows && !(x1 < wx0 + 0 || x0 > wx0 + 3));
-                    m1 = __ballot_sync(FULL_MASK, rows && !(x1 < wx0 + 4 || x0 > wx0 + 7));
-                    m2 = __ballot_sync(FULL_MASK, rows && !(x1 < wx0 + 8 || x0 > wx0 + 11));
-                    m3 = __ballot_sync(FULL_MASK, rows && !(x1 < wx0 + 12 || x0 > wx0 + 15));
                 }
-                uint32_t mine = grp == 0 ? m0 : (grp == 1 ? m1 : (grp == 2 ? m2 : m3));
-                // every lane runs every iteration (no early exits) so the group reductions are legal
-                while (__any_sync(FULL_MASK, mine != 0u)) {
-                    const bool have = mine != 0u;
-                    const uint32_t j = have ? j0 + (uint32_t)(__ffs(mine) - 1) : 0u;
-                    if (have) mine &= mine - 1u;
-                    float g[GR];
 #pragma unroll
-                    for (int k = 0; k < GR; ++k) g[k] = 0.0f;
-                    bool contrib = false;
-                    if (have && !done) {
-                        const float4 q1 = s_q1[j], q2 = s_q2[j];
-                        const uint32_t lo = __float_as_uint(q1.w), hi = __float_as_uint(q2.w);
-                        const int x0 = (int)(lo & 0xFFFFu), y0 = (int)(lo >> 16);
-                        const int x1 = (int)(hi & 0xFFFFu), y1 = (int)(hi >> 16);
-                        if ((unsigned)(px - x0) <= (unsigned)(x1 - x0) && (unsigned)(py - y0) <= (unsigned)(y1 - y0)) {
-                            const float4 q0 = s_q0[j];
-                            const float tcx = fmaf(q0.y, Y, fmaf(q0.x, X, q0.z));
-                            const float tcy = fmaf(q1.x, Y, fmaf(q0.w, X, q1.y));
-                            bool cov;
-                            if (RECT) {
-                                cov = fabsf(tcx) <= margin && fabsf(tcy) <= margin;
-                            } else {
-                                const float4 q3 = s_q3[j];
-                                const float dx = fmaf(psx, X, q3.x), dy = fmaf(psy, Y, q3.y);
-                                cov = fabsf(dx) <= q3.z && fabsf(dy) <= q3.z;
+                for (uint32_t q = 0; q < 8u; ++q) {
+                    count = grp == q ? n[q] : count;
+                    longest = max(longest, n[q]);
+                }
+                __syncwarp();
+            }
+            // every lane runs every iteration (no early exits) so the group reductions are legal
+            for (uint32_t k = 0; k < longest; ++k) {
+                uint32_t j = 0u;
+                bool contrib = false;
+                float g[GR];
+#pragma unroll
+                for (int m = 0; m < GR; ++m) g[m] = 0.0f;
+                if (k < count) {
+                    j = s_list[w][grp][k];
+                    if (!done && (s_pm[w][j] & my_pixel) != 0u) {
+                        const float4 qa = s_a[j], qb = s_b[j];
+                        const float2 tc = fma2(make_float2(qa.z, qa.w), make_float2(Y, Y),
+                                               fma2(make_float2(qa.x, qa.y), make_float2(X, X), make_float2(qb.x, qb.y)));
+                        bool cov;
+                        if (RECT) {
+                            cov = fabsf(tc.x) <= margin && fabsf(tc.y) <= margin;
+                        } else {
+                            const float4 q3 = s_q3[j];
+                            const float dx = fmaf(psx, X, q3.x), dy = fmaf(psy, Y, q3.y);
+                            cov = fabsf(dx) <= q3.z && fabsf(dy) <= q3.z;
+                        }
+                        const float power = fmaf(tc.x, tc.x, tc.y * tc.y);
+                        const float a = qb.z;
+                        float E = 0.0f, alpha = 0.0f;
+                        if (cov) {
+                            E = spl_expf_falloff<FAR>(-0.5f * power);
+                            alpha = a * E;
+                        }
+                        if (cov && !(alpha < alpha_min)) {
+                            contrib = true;
+                            const float4 qc = s_c[j];
+                            const float rgb[3] = {qb.w, qc.x, qc.y};
+                            float s[3], dS[3];
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) {
+                                s[c] = __saturatef(rgb[c] * alpha);
+                                dS[c] = gC[c] * T;
+                                Ca[c] = s[c] * T + Ca[c];  // the forward's operation order
                             }
-                            if (cov) {
-                                const float power = fmaf(tcx, tcx, tcy * tcy);
-                                const float E = spl_expf_falloff<true>(-0.5f * power);
-                                const float a = q1.z;
-                                const float alpha = a * E;
-                                if (!(alpha < alpha_min)) {
-                                    contrib = true;
-                                    const float rgb[3] = {q2.x, q2.y, q2.z};
-                                    float s[3], dS[3];
-                                    const float sa = __saturatef(alpha);
+                            const float om = 1.0f - __saturatef(alpha);
+                            float dsa = 0.0f;
+                            if (om > 0.0f) {  // om in (0, 1]: the fast divide is within 2 ulp
+                                const float Sdot =
+                                    (gC[0] * (Cf[0] - Ca[0]) + gC[1] * (Cf[1] - Ca[1])) + gC[2] * (Cf[2] - Ca[2]);
+                                dsa = __fdividef(-(Sdot + kT), om);
+                            }
+                            T = T * om;
+                            done = T < FP32_T_MIN;
+                            float dalpha = alpha < 1.0f ? dsa : 0.0f;
 #pragma unroll
-                                    for (int c = 0; c < 3; ++c) {
-                                        s[c] = __saturatef(rgb[c] * alpha);
-                                        dS[c] = gC[c] * T;
-                                        Ca[c] = s[c] * T + Ca[c];  // the forward's operation order
-                                    }
-                                    const float om = 1.0f - sa;
-                                    float dsa = 0.0f;
-                                    if (om > 0.0f) {  // om in (0, 1]: the fast divide is within 2 ulp
-                                        const float Sdot =
-                                            (gC[0] * (Cf[0] - Ca[0]) + gC[1] * (Cf[1] - Ca[1])) + gC[2] * (Cf[2] - Ca[2]);
-                                        dsa = __fdividef(-(Sdot + kT), om);
-                                    }
-                                    T = T * om;
-                                    done = T < FP32_T_MIN;
-                                    float dalpha = alpha < 1.0f ? dsa : 0.0f;
-#pragma unroll
-                                    for (int c = 0; c < 3; ++c) {
-                                        const float v = rgb[c] * alpha;
-                                        if (v > 0.0f && v < 1.0f) {
-                                            dalpha += dS[c] * rgb[c];
-                                            g[7 + c] = dS[c] * alpha;
-                                        }
-                                    }
-                                    g[6] = dalpha * E;
-                                    const float dpow = -0.5f * (dalpha * a * E);
-                                    const float dtx = 2.0f * dpow * tcx, dty = 2.0f * dpow * tcy;
-                                    // A against offsets from the box centre (Xr, Yr), B at that centre
-                                    const float ox = X - 0.5f * (float)(x0 + x1 + 1);
-                                    const float oy = Y - 0.5f * (float)(y0 + y1 + 1);
-                                    g[0] = dtx * ox;
-                                    g[1] = dtx * oy;
-                                    g[2] = dtx;
-                                    g[3] = dty * ox;
-                                    g[4] = dty * oy;
-                                    g[5] = dty;
+                            for (int c = 0; c < 3; ++c) {
+                                if (s[c] > 0.0f && s[c] < 1.0f) {  // the clamp passes it on
+                                    dalpha += dS[c] * rgb[c];
+                                    g[7 + c] = dS[c] * alpha;
                                 }
                             }
+                            g[6] = dalpha * E;
+                            const float dpow = -0.5f * (dalpha * a * E);
+                            const float dtx = 2.0f * dpow * tc.x, dty = 2.0f * dpow * tc.y;
+                            // A against offsets from the box centre (Xr, Yr), B at that centre
+                            const float ox = X - qc.z, oy = Y - qc.w;
+                            g[0] = dtx * ox;
+                            g[1] = dtx * oy;
+                            g[2] = dtx;
+                            g[3] = dty * ox;
+                            g[4] = dty * oy;
+                            g[5] = dty;
                         }
                     }
-                    // reduce over the 8 lanes of the group (all hold the same record this iteration)
-                    const uint32_t gm = __ballot_sync(FULL_MASK, contrib);
-                    if (gm != 0u) {
-                        float v0, v1;
-                        const uint32_t k0 = reduce10_over8(g, li, v0, v1);
-                        if ((gm >> (grp * 8u)) & 0xFFu) {
-                            float* dst = grad_rec + (size_t)s_slot[j] * GR;
-                            atomicAdd(dst + k0, v0);
-                            if ((li & 3u) == 0u) atomicAdd(dst + k0 + 1u, v1);
-                        }
+                }
+                // reduce over the lanes of the group (all hold the same record this iteration)
+                const uint32_t gm = __ballot_sync(FULL_MASK, contrib);
+                if (gm != 0u) {
+                    float v[3];
+                    const uint32_t k0 = reduce10_over4(g, li, v);
+                    if ((gm >> (grp * 4u)) & 0xFu) {
+                        float* dst = grad_rec + (size_t)s_row[j] * GR + k0;
+                        atomicAdd(dst, v[0]);
+                        atomicAdd(dst + 1, v[1]);
+                        if (!(li & 1u)) atomicAdd(dst + 2, v[2]);
                     }
                 }
             }
@@ -382,12 +387,10 @@ void launch_backward(int sh_order, bool covariance, bool rect, const SceneView& 
     k_zero_grad_rec<<<zg, 256, 0, st>>>(grad_rec, fc, deferred);
     const int grid = tiles_x * tiles_y;
     if (grid > 0) {
-        if (rect)
-            k_raster_backward<true><<<grid, 256, 0, st>>>(ranges, tile_order, pair_vals, rec, W, H, tiles_x, u.margin,
-                                                          psx, psy, image, grad_image, grad_rec);
-        else
-            k_raster_backward<false><<<grid, 256, 0, st>>>(ranges, tile_order, pair_vals, rec, W, H, tiles_x,
-                                                           u.margin, psx, psy, image, grad_image, grad_rec);
+        auto k = !rect ? k_raster_backward<false, true>
+                       : (fabsf(u.margin) <= RASTER_NEAR_MARGIN ? k_raster_backward<true, false> : k_raster_backward<true, true>);
+        k<<<grid, 256, 0, st>>>(ranges, tile_order, pair_vals, rec, W, H, tiles_x, u.margin, psx, psy, image, grad_image,
+                                grad_rec);
     }
     if (max_n == 0) return;
     uint32_t blocks = (max_n + 127) / 128;

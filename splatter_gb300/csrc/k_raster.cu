@@ -14,7 +14,7 @@
 //                    batches of 256, per-pixel record lists from the boxes (bit-transposed ballots),
 //                    exact coverage test, falloff, blend, and early exit once every pixel of the tile
 //                    is opaque
-#include "spl_device.cuh"
+#include "spl_raster.cuh"
 
 namespace spl {
 
@@ -308,9 +308,6 @@ __global__ void __launch_bounds__(1024) k_tile_order(const uint2* __restrict__ r
 }
 
 // ------------------------------------------------------------------------------------------------
-constexpr int RASTER_BATCH = 256;
-constexpr int RASTER_WORDS = RASTER_BATCH / 32;
-constexpr float RASTER_NEAR_MARGIN = 9.0f;  // up to this margin a covered pixel's exponent stays above -87
 
 // One CTA per 16x16 tile, one thread per pixel.  Warp w owns the strip of rows 2w, 2w+1; lane l holds
 // column l & 15 and row 2w + l / 16.  The tile's records (depth order) are staged through shared memory in batches of 256,
@@ -334,33 +331,6 @@ constexpr float RASTER_NEAR_MARGIN = 9.0f;  // up to this margin a covered pixel
 //   (without the packed pairs 417 and 1,062 us).
 // Batches of 512 records (fewer, longer walks) lose more to the fewer resident CTAs: 483 us; five CTAs per
 // SM at 48 registers, without spills: 416 us.
-
-// Two float operations per instruction on packed pairs (the results of the scalar operations, each rounded
-// to nearest).  The assembler contracts a packed product and a packed sum that takes it into a packed fma
-// even where plain contraction is off, so a product that is to be rounded before a sum is a product with a
-// zero addend (fma2, the same value for a non-negative product) or its sum is scalar.
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 d;
-    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mul.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 d;
-    asm("{.reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; add.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d;}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{.reg .b64 a, b, c, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mov.b64 c, {%6, %7}; "
-        "fma.rn.f32x2 d, a, b, c; mov.b64 {%0, %1}, d;}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
 
 // The unorm8 value nearest to v in [0, 1] (k / 255, k = v * 255 rounded to nearest even), as the float
 // nearest to k / 255: adding 2^23 leaves the integer k in the mantissa's last bits, and k / 255 is the
@@ -398,18 +368,6 @@ __device__ __forceinline__ void transpose_lane_bits_n(uint32_t* x, uint32_t lane
             x[c] = (x[c] & keep) | (__funnelshift_l(p, p, rot) & ~keep);
         }
     }
-}
-
-// Highest set bit of x (x != 0).
-__device__ __forceinline__ uint32_t top_bit(uint32_t x) {
-    uint32_t r;
-    asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(x));
-    return r;
-}
-
-// Columns a .. b - 1 of a row of 16 as a bit mask (a, b <= 16, in their low five bits; empty when a >= b).
-__device__ __forceinline__ uint32_t row_columns(uint32_t a, uint32_t b) {
-    return __funnelshift_l(0u, 0xFFFFu, a) & ~__funnelshift_l(0u, 0xFFFFFFFFu, b) & 0xFFFFu;
 }
 
 // FAR: a covered pixel's exponent may fall below -87 (axis-aligned squares, or a margin above
@@ -451,57 +409,7 @@ __global__ void __launch_bounds__(256, 6) k_raster(const uint2* __restrict__ ran
             s_b[slot] = make_float4(r0.z, r1.y, r1.z, r2.x);
             s_c[slot] = make_float2(r2.y, r2.z);
             if (!RECT) s_q3[slot] = __ldg(r + 3);
-            // The record's lane mask for each of the tile's eight strips (rows 2w, 2w + 1), one 16-bit half
-            // per row: the pixels inside its pixel box and, for rectangles, only those whose centre may lie in
-            // the rectangle: along a row tc is c + x A, so |c + x A| <= T is the interval (-c +- T) / A of
-            // columns x.  T is the margin widened by a rounding bound far above the errors of the
-            // per-pixel FMA chains and of this arithmetic (1e-6 of each term of c and of T itself), the
-            // interval by another 1e-3 columns.  Pixels left out are not drawn by the record: the image
-            // is unchanged.
-            const uint32_t lo = __float_as_uint(r1.w), hi = __float_as_uint(r2.w);
-            const int x0 = (int)(lo & 0xFFFFu), y0 = (int)(lo >> 16);
-            const int x1 = (int)(hi & 0xFFFFu), y1 = (int)(hi >> 16);
-            if (x0 <= x1 && y0 <= y1) {
-                const int ty0 = ty * TILE_PIXELS;
-                const int ra = max(y0 - ty0, 0), rb = min(y1 - ty0, 15);  // the box's rows and columns here
-                const uint32_t box = row_columns((uint32_t)max(x0 - wx0, 0), (uint32_t)min(x1 - wx0, 15) + 1u);
-                float2 c = make_float2(0.0f, 0.0f), step = c, half = make_float2(1e9f, 1e9f);
-                if (RECT) {
-                    // column 0 of row ra; row after row the interval's centre moves by step
-                    const float Xc = (float)wx0 + 0.5f, Yc = (float)(ty0 + ra) + 0.5f;
-                    const float Xm = (float)(wx0 + 16), Ym = (float)(ty0 + 16);
-                    if (fabsf(r0.x) > 1e-30f) {
-                        const float s = -1.0f / r0.x;
-                        const float T = margin + 1e-6f * (fabsf(r0.x) * Xm + fabsf(r0.y) * Ym + fabsf(r0.z) + margin);
-                        c.x = fmaf(r0.y, Yc, fmaf(r0.x, Xc, r0.z)) * s;
-                        step.x = r0.y * s;
-                        half.x = T * fabsf(s) + 1e-3f;
-                    }
-                    if (fabsf(r0.w) > 1e-30f) {
-                        const float s = -1.0f / r0.w;
-                        const float T = margin + 1e-6f * (fabsf(r0.w) * Xm + fabsf(r1.x) * Ym + fabsf(r1.y) + margin);
-                        c.y = fmaf(r1.x, Yc, fmaf(r0.w, Xc, r1.y)) * s;
-                        step.y = r1.x * s;
-                        half.y = T * fabsf(s) + 1e-3f;
-                    }
-                }
-                uint16_t* pm = reinterpret_cast<uint16_t*>(&s_pm[0][slot]);
-                for (int row = ra; row <= rb; ++row) {
-                    uint32_t m = box;
-                    if (RECT) {
-                        const float k = (float)(row - ra);
-                        const float2 q = fma2(make_float2(k, k), step, c);
-                        const float2 qa = add2(q, make_float2(-half.x, -half.y)), qb = add2(q, half);
-                        // first column: the bound rounded up; one past the last: rounded down, plus one
-                        const float fa = fminf(fmaxf(fmaxf(qa.x, qa.y), 0.0f), 16.0f);
-                        const float fb = fmaxf(fminf(fminf(qb.x, qb.y), 15.0f), -1.0f);
-                        m &= row_columns(__float_as_uint(__fadd_ru(fa, 8388608.0f)),
-                                         __float_as_uint(__fadd_rd(fb, 8388609.0f)));
-                    }
-                    // strip row / 2, half row & 1
-                    pm[(row >> 1) * (2 * RASTER_BATCH) + (row & 1)] = (uint16_t)m;
-                }
-            }
+            mask_rows<RECT>(s_pm, slot, r0, r1, r2, wx0, ty * TILE_PIXELS, margin);
         }
         __syncthreads();
         if (!warp_done) {
