@@ -258,8 +258,8 @@ int spl_renderer_create(const spl_config* cfg, spl_renderer** out) {
     TRY(dalloc(&r->idx, n));
     TRY(dalloc(&r->rec, n * 4));
     TRY(dalloc(&r->boxes, n));
-    TRY(dalloc(&r->st_cull, ceil_div(n, CULL_TILE)));
-    TRY(dalloc(&r->st_bin, ceil_div(n, BIN_TILE)));
+    TRY(dalloc(&r->st_cull, LB_LINE * ceil_div(n, CULL_TILE_SMALL)));
+    TRY(dalloc(&r->st_bin, LB_LINE * ceil_div(n, BIN_TILE)));
     TRY(dalloc(&r->pk_a, pc));
     TRY(dalloc(&r->pk_b, pc));
     TRY(dalloc(&r->pv_a, pc));
@@ -274,8 +274,8 @@ int spl_renderer_create(const spl_config* cfg, spl_renderer** out) {
 #undef TRY
     cudaError_t e = cudaSuccess;
     // status words start at epoch 0, which no frame uses
-    if (e == cudaSuccess) e = cudaMemset(r->st_cull, 0, ceil_div(n, CULL_TILE) * 8);
-    if (e == cudaSuccess) e = cudaMemset(r->st_bin, 0, ceil_div(n, BIN_TILE) * 8);
+    if (e == cudaSuccess) e = cudaMemset(r->st_cull, 0, LB_LINE * ceil_div(n, CULL_TILE_SMALL) * 8);
+    if (e == cudaSuccess) e = cudaMemset(r->st_bin, 0, LB_LINE * ceil_div(n, BIN_TILE) * 8);
     if (e == cudaSuccess) e = cudaMemset(r->fc, 0, sizeof(FrameCounters));
     if (e == cudaSuccess) e = cudaMemset(r->fc_sort, 0, sizeof(FrameCounters));
     if (e == cudaSuccess)
@@ -341,7 +341,7 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
         // four stable 8-bit passes a -> b -> a -> b -> a; pass 0 takes the compaction slot as the value
         if (coop) {
             CU(launch_sort_coop(r->keys_a, r->keys_b, r->vals_a, r->vals_b, true, &r->fc->visible, N, 4, 0,
-                                r->coop_table, r->epoch, r->fc->barrier, sl, &r->fc->err, st));
+                                r->coop_table, r->epoch, &r->fc->barrier[0].v, sl, &r->fc->err, st));
         } else {
             // digit histograms from the cull kernel; one launch per pass
             uint32_t *src_k = r->keys_a, *dst_k = r->keys_b, *dst_v = r->vals_b;
@@ -349,7 +349,7 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
             const uint64_t stride = r->sort_tiles() * 256;
             for (int p = 0; p < 4; ++p) {
                 launch_onesweep(src_k, src_v, dst_k, dst_v, &r->fc->visible, N, r->fc->hist_depth[p],
-                                r->st_sort + p * stride, &r->fc->tile_counter[1 + p], r->epoch, 8 * p, sl,
+                                r->st_sort + p * stride, &r->fc->tile_counter[1 + p].v, r->epoch, 8 * p, sl,
                                 &r->fc->err, st);
                 uint32_t* next_k = dst_k == r->keys_b ? r->keys_a : r->keys_b;
                 uint32_t* next_v = dst_v == r->vals_b ? r->vals_a : r->vals_b;
@@ -369,14 +369,14 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
     const int passes = tiles <= 256 ? 1 : (tiles <= 65536 ? 2 : 3);
     if (coop) {
         CU(launch_sort_coop(r->pk_a, r->pk_b, r->pv_a, r->pv_b, false, &r->fc->pairs, (uint32_t)r->pair_cap, passes,
-                            0, r->coop_table + sort_coop_table_words(), r->epoch, r->fc->barrier + 1, sl, &r->fc->err, st));
+                            0, r->coop_table + sort_coop_table_words(), r->epoch, &r->fc->barrier[1].v, sl, &r->fc->err, st));
     } else {
         // tile-id histograms from the binning kernel
         uint32_t *ak = r->pk_a, *av = r->pv_a, *bk = r->pk_b, *bv = r->pv_b;
         const uint64_t pstride = r->pair_tiles() * 256;
         for (int p = 0; p < passes; ++p) {
             launch_onesweep(ak, av, bk, bv, &r->fc->pairs, (uint32_t)r->pair_cap, r->fc->hist_pairs[p],
-                            r->st_pairs + p * pstride, &r->fc->tile_counter[5 + p], r->epoch, 8 * p, sl, &r->fc->err,
+                            r->st_pairs + p * pstride, &r->fc->tile_counter[5 + p].v, r->epoch, 8 * p, sl, &r->fc->err,
                             st);
             std::swap(ak, bk);
             std::swap(av, bv);
@@ -627,7 +627,7 @@ int spl_sort_pairs(spl_renderer* r, const uint32_t* keys_in, const uint32_t* val
     CU(cudaMemcpyAsync(r->keys_a, keys_in, count * 4, cudaMemcpyDeviceToDevice, st));
     CU(cudaMemcpyAsync(r->vals_a, values_in, count * 4, cudaMemcpyDeviceToDevice, st));
     CU(launch_sort_coop(r->keys_a, r->keys_b, r->vals_a, r->vals_b, false, &r->fc_sort->visible, (uint32_t)count,
-                        passes, 0, r->coop_table, r->epoch, r->fc_sort->barrier, r->spin_limit, &r->fc_sort->err, st));
+                        passes, 0, r->coop_table, r->epoch, &r->fc_sort->barrier[0].v, r->spin_limit, &r->fc_sort->err, st));
     const uint32_t* kr = (passes & 1) ? r->keys_b : r->keys_a;
     const uint32_t* vr = (passes & 1) ? r->vals_b : r->vals_a;
     CU(cudaMemcpyAsync(keys_out, kr, count * 4, cudaMemcpyDeviceToDevice, st));

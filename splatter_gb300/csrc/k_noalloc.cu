@@ -100,7 +100,7 @@ extern "C" int spl_sort_pairs_no_alloc(const uint32_t* keys_in, const uint32_t* 
         uint32_t* kout = to_out ? keys_out : s->tmp_keys;
         uint32_t* vout = to_out ? values_out : s->tmp_vals;
         launch_onesweep(kin, vin, kout, vout, &s->fc.visible, (uint32_t)count, s->fc.hist_depth[p], s->status[p],
-                        &s->fc.tile_counter[1 + p], &s->epoch, 8 * p, 1u << 20, &s->fc.err, st);
+                        &s->fc.tile_counter[1 + p].v, &s->epoch, 8 * p, 1u << 20, &s->fc.err, st);
         kin = kout;
         vin = vout;
     }

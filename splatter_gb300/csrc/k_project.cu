@@ -18,9 +18,8 @@ namespace spl {
 
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void counters_begin(FrameCounters* fc, uint32_t* epoch_word) {
-    uint32_t* w = reinterpret_cast<uint32_t*>(fc);
-    const uint32_t nwords = sizeof(FrameCounters) / 4;
-    for (uint32_t i = threadIdx.x; i < nwords; i += blockDim.x) w[i] = 0u;
+    uint4* w = reinterpret_cast<uint4*>(fc);
+    for (uint32_t i = threadIdx.x; i < sizeof(FrameCounters) / 16; i += blockDim.x) w[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t e = *epoch_word + 1u;
@@ -68,11 +67,15 @@ __device__ __forceinline__ void stage_frame(const Uniforms* __restrict__ d_u, Un
 }
 
 // ------------------------------------------------------------------------------------------------
-// Cull + key + histogram + ordered compaction.  One CTA handles 4096 consecutive splats; warp w owns
-// splats [w*512, w*512+512) of the tile and lane l handles elements w*512 + 32*j + l, so loads are
-// coalesced and the ballot order is the index order.
-template <int MODE, bool HIST>
-__global__ void __launch_bounds__(256, 3) k_cull_key(const SceneView* __restrict__ d_sv, const Uniforms* __restrict__ d_u,
+// Cull + key + histogram + ordered compaction.  One CTA handles a tile of 256 x PER_LANE consecutive splats; warp w
+// owns an eighth of the tile and lane l handles its elements 32*j + l, so loads are coalesced and the ballot
+// order is the index order.
+// Bound by latency: the ticket and the uniform block, the loads, some 120 instructions per splat, the look-back.
+// 6M splats 66 -> 50 us (look-back words in lines of their own and 256 of them per step: 52 us; tiles of 2048 splats
+// instead of 4096, four CTAs per SM: 50 us, tiles of 1024: 61 us), 1M 26 -> 21 us; frames of up to 2^19 splats,
+// which fit one wave in tiles of 1024, take those: 100k 18 -> 15 us, 350k 19 -> 16 us.
+template <int MODE, bool HIST, int PER_LANE>
+__global__ void __launch_bounds__(256, 4) k_cull_key(const SceneView* __restrict__ d_sv, const Uniforms* __restrict__ d_u,
                                                   FrameCounters* fc,
                                                   const uint32_t* __restrict__ epoch_word, uint64_t* status,
                                                   uint32_t* __restrict__ keys_out, uint32_t* __restrict__ idx_out,
@@ -88,18 +91,18 @@ __global__ void __launch_bounds__(256, 3) k_cull_key(const SceneView* __restrict
     frame_step(d_sv, d_u, epoch_word);
     stage_frame(d_u, s_u, d_sv, s_sv);
     if (tid == 0) {
-        s_tile = atomicAdd(&fc->tile_counter[0], 1u);
+        s_tile = atomicAdd(&fc->tile_counter[0].v, 1u);
         s_epoch = *epoch_word;
     }
     __syncthreads();
     const Uniforms& u = s_u;
     const SceneView& s = s_sv;
     const uint32_t tile = s_tile, epoch = s_epoch, n = s.n;
-    const uint32_t ntiles = (n + CULL_TILE - 1) / CULL_TILE;
+    constexpr uint32_t TILE = 256u * PER_LANE;
+    const uint32_t ntiles = (n + TILE - 1) / TILE;
     if (tile >= ntiles) return;  // a grid sized for a larger scene (captured frames)
-    const uint32_t base = tile * CULL_TILE + w * (CULL_TILE / 8u) + lane;
+    const uint32_t base = tile * TILE + w * (TILE / 8u) + lane;
 
-    constexpr int PER_LANE = CULL_TILE / 256;
     float px[PER_LANE], py[PER_LANE], pz[PER_LANE];
 #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) {
@@ -166,10 +169,10 @@ __global__ void __launch_bounds__(256, 3) k_cull_key(const SceneView* __restrict
         ttot += c;
     }
     if (w == 0) {
-        if (lane == 0) lb_store(status + tile, lb_pack(epoch, tile == 0 ? LB_INC : LB_AGG, ttot));
-        const uint32_t excl = tile == 0 ? 0u : lookback_single(status, tile, epoch, spin_limit, &fc->err);
+        if (lane == 0) lb_store(status + lb_word(tile), lb_pack(epoch, tile == 0 ? LB_INC : LB_AGG, ttot));
+        const uint32_t excl = lookback_single<8>(status, tile, epoch, spin_limit, &fc->err);
         if (lane == 0) {
-            if (tile != 0) lb_store(status + tile, lb_pack(epoch, LB_INC, excl + ttot));
+            if (tile != 0) lb_store(status + lb_word(tile), lb_pack(epoch, LB_INC, excl + ttot));
             s_base = excl;
             if (tile == ntiles - 1) fc->visible = excl + ttot;
         }
@@ -200,9 +203,13 @@ void launch_cull_key(int mode, bool hist, uint32_t grid_n, const SceneView* d_sv
                      FrameCounters* fc, const uint32_t* epoch_word, uint64_t* status, uint32_t* keys_out,
                      uint32_t* idx_out, uint32_t spin_limit, cudaStream_t st) {
     if (grid_n == 0) return;
-    const uint32_t grid = (grid_n + CULL_TILE - 1) / CULL_TILE;
-    auto k = mode == DS_CPU ? (hist ? k_cull_key<DS_CPU, true> : k_cull_key<DS_CPU, false>)
-                            : (hist ? k_cull_key<DS_GPU, true> : k_cull_key<DS_GPU, false>);
+    const bool small = grid_n <= CULL_SMALL_MAX;
+    const uint32_t tile = small ? CULL_TILE_SMALL : CULL_TILE, grid = (grid_n + tile - 1) / tile;
+    constexpr int L = CULL_TILE / 256, S = CULL_TILE_SMALL / 256;
+    auto k = mode == DS_CPU ? (hist ? (small ? k_cull_key<DS_CPU, true, S> : k_cull_key<DS_CPU, true, L>)
+                                    : (small ? k_cull_key<DS_CPU, false, S> : k_cull_key<DS_CPU, false, L>))
+                            : (hist ? (small ? k_cull_key<DS_GPU, true, S> : k_cull_key<DS_GPU, true, L>)
+                                    : (small ? k_cull_key<DS_GPU, false, S> : k_cull_key<DS_GPU, false, L>));
     launch_after(k, grid, 256, st, d_sv, u, fc, epoch_word, status, keys_out, idx_out, spin_limit);
 }
 
@@ -490,7 +497,7 @@ void launch_gather_entries(const uint32_t* keys, const uint32_t* slots, const ui
 // publishes (status[0] is never written).  The wait runs out after spin_limit polls, raises the
 // error bit and returns; out[0] = prefix it gave up with, out[1] = error word.
 __global__ void k_lookback_probe(uint64_t* status, uint32_t* err, uint32_t spin_limit, uint32_t* out) {
-    const uint32_t excl = lookback_single(status, 1u, 7u, spin_limit, err);
+    const uint32_t excl = lookback_single<8>(status, 1u, 7u, spin_limit, err);
     __syncwarp();
     if (threadIdx.x == 0) {
         out[0] = excl;

@@ -19,9 +19,10 @@
 namespace spl {
 
 // ------------------------------------------------------------------------------------------------
+constexpr int BIN_LB = 2, BIN_CTAS = 6;
 constexpr int BIN_PER = BIN_TILE / 256;  // consecutive draw entries per thread (thread order = depth order)
 template <bool ORDERED, bool HIST>
-__global__ void __launch_bounds__(256) k_bin(const uint32_t* __restrict__ order, const uint2* __restrict__ boxes,
+__global__ void __launch_bounds__(256, BIN_CTAS) k_bin(const uint32_t* __restrict__ order, const uint2* __restrict__ boxes,
                                              FrameCounters* fc, int mode, const uint32_t* __restrict__ epoch_word,
                                              uint64_t* status, uint32_t* __restrict__ pair_keys,
                                              uint32_t* __restrict__ pair_vals, uint32_t pair_cap, int tiles_x,
@@ -39,7 +40,7 @@ __global__ void __launch_bounds__(256) k_bin(const uint32_t* __restrict__ order,
     // every tile's range starts empty
     for (uint32_t i = blockIdx.x * 256u + tid; i < tiles; i += gridDim.x * 256u) ranges[i] = make_uint2(0u, 0u);
     if (tid == 0) {
-        s_tile = atomicAdd(&fc->tile_counter[8], 1u);
+        s_tile = atomicAdd(&fc->tile_counter[8].v, 1u);
         s_epoch = *epoch_word;
         const uint32_t V = fc->visible;
         uint32_t draw = V;
@@ -96,10 +97,10 @@ __global__ void __launch_bounds__(256) k_bin(const uint32_t* __restrict__ order,
         off += cnt[e];
     }
     if (tid < 32) {
-        if (tid == 0) lb_store(status + tile, lb_pack(epoch, tile == 0 ? LB_INC : LB_AGG, btot));
-        const uint32_t excl = tile == 0 ? 0u : lookback_single(status, tile, epoch, spin_limit, &fc->err);
+        if (tid == 0) lb_store(status + lb_word(tile), lb_pack(epoch, tile == 0 ? LB_INC : LB_AGG, btot));
+        const uint32_t excl = lookback_single<BIN_LB>(status, tile, epoch, spin_limit, &fc->err);
         if (tid == 0) {
-            if (tile != 0) lb_store(status + tile, lb_pack(epoch, LB_INC, excl + btot));
+            if (tile != 0) lb_store(status + lb_word(tile), lb_pack(epoch, LB_INC, excl + btot));
             s_base = excl;
             if (tile == ntiles - 1) {
                 fc->pairs = excl + btot;

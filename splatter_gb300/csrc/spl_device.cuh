@@ -73,44 +73,59 @@ __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t* p) {
     return v;
 }
 
-// Warp-cooperative look-back for a single running total (stream compaction, bin offsets).
-// Called by all 32 lanes of one warp; returns the exclusive prefix of `tile` (sum of all earlier
-// tiles).  Every wait is bounded: after spin_limit polls the error flag is raised and the missing
-// predecessors count as zero, so the kernel always terminates.
+// Look-back for a single running total (stream compaction, bin offsets), called by all 32 lanes of one warp;
+// returns the exclusive prefix of `tile` (sum of all earlier tiles): 32 x WORDS words at a time, down to the nearest
+// inclusive prefix.  The steps are a chain of L2 round trips, so a step is wide where the registers allow it; and
+// every tile's word has a line of its own (lb_word): the tiles of a wave publish and wait at the same time, and
+// stores to a line that many others read cost some 20 ns each.  With 16 words to a line a wait of 245 tiles
+// whose predecessors had all published took 6-7 us instead of 1.
+// Every wait is bounded: after spin_limit polls, or once another wait has run out, the error flag is raised and the
+// missing predecessors count as zero, so the kernel always terminates.
+__device__ __forceinline__ size_t lb_word(size_t tile) { return tile * LB_LINE; }
+template <int WORDS>
 __device__ __forceinline__ uint32_t lookback_single(const uint64_t* status, uint32_t tile, uint32_t epoch,
                                                     uint32_t spin_limit, uint32_t* err) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t excl = 0;
-    int64_t window = (int64_t)tile - 1;
-    while (window >= 0) {
-        const int64_t idx = window - (int64_t)lane;
-        uint64_t s = 0;
-        uint32_t ready_mask = 0, inc_mask = 0, need = 0;
-        uint32_t spins = 0;
-        bool timed_out = false;
+    for (uint32_t end = tile; end > 0u; end -= 32u * WORDS) {
+        uint64_t v[WORDS];
+#pragma unroll
+        for (uint32_t j = 0; j < (uint32_t)WORDS; ++j) {
+            const uint32_t off = lane + 32u * j;
+            v[j] = off < end ? lb_load(status + lb_word(end - 1u - off)) : lb_pack(epoch, LB_INC, 0);
+        }
+        uint32_t nearest, spins = 0;
         for (;;) {
-            s = idx >= 0 ? lb_load(status + idx) : lb_pack(epoch, LB_INC, 0);
-            const bool ready = (uint32_t)(s >> 32) == epoch && ((uint32_t)s & (LB_AGG | LB_INC)) != 0;
-            const bool inc = ready && ((uint32_t)s & LB_INC) != 0;
-            ready_mask = __ballot_sync(FULL_MASK, ready);
-            inc_mask = __ballot_sync(FULL_MASK, inc);
-            const int stop = inc_mask ? __ffs(inc_mask) - 1 : 31;
-            need = stop == 31 ? FULL_MASK : ((2u << stop) - 1u);
-            if ((ready_mask & need) == need) break;
-            if (++spins > spin_limit) {
-                timed_out = true;
-                break;
+            nearest = 0xFFFFFFFFu;
+            uint32_t first_missing = 0xFFFFFFFFu;
+#pragma unroll
+            for (uint32_t j = 0; j < (uint32_t)WORDS; ++j) {
+                const uint32_t off = lane + 32u * j, f = (uint32_t)v[j];
+                const bool ready = (uint32_t)(v[j] >> 32) == epoch && (f & (LB_AGG | LB_INC)) != 0u;
+                if (ready && (f & LB_INC) != 0u) nearest = min(nearest, off);
+                if (!ready) first_missing = min(first_missing, off);
             }
-            if (spins > 16) __nanosleep(64);
+            nearest = __reduce_min_sync(FULL_MASK, nearest);
+            if (__reduce_min_sync(FULL_MASK, first_missing) > nearest ||
+                (nearest == 0xFFFFFFFFu && __all_sync(FULL_MASK, first_missing == 0xFFFFFFFFu)))
+                break;
+            if (++spins > spin_limit || ((spins & 1023u) == 0u && (ld_relaxed_u32(err) & SPL_DEV_ERR_LOOKBACK))) {
+                if (lane == 0u) atomicOr(err, SPL_DEV_ERR_LOOKBACK);
+                return excl;
+            }
+            if (spins > 4u) __nanosleep(40);
+#pragma unroll
+            for (uint32_t j = 0; j < (uint32_t)WORDS; ++j) {
+                const uint32_t off = lane + 32u * j;
+                const bool ready = (uint32_t)(v[j] >> 32) == epoch && ((uint32_t)v[j] & (LB_AGG | LB_INC)) != 0u;
+                if (!ready && off <= nearest) v[j] = lb_load(status + lb_word(end - 1u - off));
+            }
         }
-        if (timed_out) {
-            if (lane == 0) atomicOr(err, SPL_DEV_ERR_LOOKBACK);
-            return excl;
-        }
-        const uint32_t v = (need >> lane) & 1u ? ((uint32_t)s & LB_VAL) : 0u;
-        excl += __reduce_add_sync(FULL_MASK, v);
-        if (inc_mask) break;
-        window -= 32;
+        uint32_t sum = 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < (uint32_t)WORDS; ++j) sum += lane + 32u * j <= nearest ? (uint32_t)v[j] & LB_VAL : 0u;
+        excl += __reduce_add_sync(FULL_MASK, sum);
+        if (nearest != 0xFFFFFFFFu) break;  // always in the window that holds the first tile
     }
     return excl;
 }

@@ -78,8 +78,8 @@ struct spl_renderer {
     uint32_t *keys_a = nullptr, *keys_b = nullptr, *vals_a = nullptr, *vals_b = nullptr, *idx = nullptr;
     float4* rec = nullptr;
     uint2* boxes = nullptr;  // pixel box of each record, for the binning kernel
-    uint64_t* st_cull = nullptr;  // [ceil(max_n/4096)]
-    uint64_t* st_bin = nullptr;   // [ceil(max_n/1024)]
+    uint64_t* st_cull = nullptr;  // [LB_LINE * ceil(max_n/1024)]
+    uint64_t* st_bin = nullptr;   // [LB_LINE * ceil(max_n/1024)]
     uint32_t *pk_a = nullptr, *pk_b = nullptr, *pv_a = nullptr, *pv_b = nullptr;
     FrameCounters* fc = nullptr;
     FrameCounters* fc_sort = nullptr;  // counters of spl_sort_pairs

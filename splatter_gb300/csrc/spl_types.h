@@ -28,9 +28,15 @@ enum : uint32_t {
     SPL_DEV_ERR_PAIR_OVERFLOW = 2u,  // the tile-binning list exceeded its capacity
 };
 
+// A word that many blocks update or wait for at once, in a 128-byte line of its own.
+struct alignas(128) HotWord {
+    uint32_t v;
+};
+
 // Per-frame counters; zeroed by k_frame_begin at the start of every frame.
 struct FrameCounters {
-    uint32_t tile_counter[12];  // dynamic tile ids: 0 cull, 1..4 depth passes, 5..7 pair passes, 8 bin
+    HotWord tile_counter[9];   // dynamic tile ids: 0 cull, 1..4 depth passes, 5..7 pair passes, 8 bin
+    HotWord barrier[2];        // grid-barrier arrivals of the cooperative depth sort and pair sort
     uint32_t visible;          // V: splats that pass the frustum test
     uint32_t keys_all_ones;    // visible splats whose composite key is 0xFFFFFFFF
     uint32_t keys_top_ff;      // visible splats whose key's top byte is 0xFF (not drawn in indirect mode)
@@ -38,7 +44,6 @@ struct FrameCounters {
     uint32_t err;              // SPL_DEV_ERR_* bits
     uint32_t draw;             // entries drawn (mode dependent)
     uint32_t epoch;            // copy of the frame epoch (for readback)
-    uint32_t barrier[2];       // grid-barrier arrivals of the cooperative depth sort and pair sort
     uint32_t hist_depth[4][256];  // digit histograms of the visible depth keys (onesweep sort only)
     uint32_t hist_pairs[3][256];  // digit histograms of the tile ids of all pairs (onesweep sort only)
 };
@@ -53,8 +58,11 @@ enum DepthSorting : int32_t { DS_NONE = 0, DS_CPU = 1, DS_GPU = 2, DS_GPU_INDIRE
 constexpr int RECORD_FLOATS = 16;
 
 constexpr int TILE_PIXELS = 16;        // raster tile edge
-constexpr int CULL_TILE = 4096;        // splats per cull/compaction tile
+constexpr int CULL_TILE = 2048;        // splats per cull/compaction tile
+constexpr int CULL_TILE_SMALL = 1024;  // the same in frames of at most CULL_SMALL_MAX splats
+constexpr uint32_t CULL_SMALL_MAX = 1u << 19;
 constexpr int SORT_TILE = 4096;        // keys per onesweep tile (256 threads x 16)
+constexpr size_t LB_LINE = 16;          // look-back status: words between one tile's and the next (128 bytes)
 constexpr int BIN_TILE = 1024;         // draw entries per binning tile (256 threads x 4)
 constexpr float FP32_T_MIN = 1e-4f;    // fp32 blend mode stops a pixel below this transmittance
 
