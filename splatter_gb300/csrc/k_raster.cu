@@ -4,9 +4,9 @@
 // destination alpha as transmittance (renderer.rs:260-271).  There is no fixed-function unit here,
 // so the frame is tiled into 16x16-pixel tiles:
 //   k_bin          - for each drawn entry in depth order, the tiles its pixel box touches; emitted as
-//                    (tile id, record slot) pairs at offsets from a decoupled look-back scan, with
-//                    load-balanced emission inside the CTA (a max-scan over the entries' first
-//                    pairs) and, for the onesweep sort, the tile-id digit histograms
+//                    (tile id, record slot) pairs at offsets from a decoupled look-back scan, emitted in
+//                    chunks of 128 pairs dealt to the CTA's warps and, for the onesweep sort, the
+//                    tile-id digit histograms
 //   (a stable radix sort of the pairs by tile id, so each tile's list stays in depth order)
 //   k_tile_ranges  - start/end of each tile's run in the sorted pair list
 //   k_tile_order   - the raster's tile order: most pairs first
@@ -19,23 +19,28 @@
 namespace spl {
 
 // ------------------------------------------------------------------------------------------------
-constexpr int BIN_LB = 2, BIN_CTAS = 6;
-constexpr int BIN_PER = BIN_TILE / 256;  // consecutive draw entries per thread (thread order = depth order)
+// Bound by latency (the ticket, the entries' boxes in a random gather, the look-back).  Emission in chunks dealt to
+// the warps instead of 1024 pairs at a time by the CTA with four barriers: 66 -> 59 us at 6M splats, 1080p, 102 -> 86
+// us at 3840x2160; tiles of 512 entries instead of 1024: 59 and 70 us, 1M splats 22 -> 16 us (tiles of 256: 14 us at
+// 1M, but 83 us at 6M, where 17k tickets at some 5 ns each set the pace; tiles of 2048: 94 us).
+constexpr int BIN_LB = 2, BIN_CTAS = 8;
+constexpr uint32_t BIN_CHUNK = 128;  // pairs that a warp emits at a time
+constexpr int BIN_PER = BIN_TILE / 256;  // consecutive draw entries per thread (depth order)
 template <bool ORDERED, bool HIST>
 __global__ void __launch_bounds__(256, BIN_CTAS) k_bin(const uint32_t* __restrict__ order, const uint2* __restrict__ boxes,
                                              FrameCounters* fc, int mode, const uint32_t* __restrict__ epoch_word,
                                              uint64_t* status, uint32_t* __restrict__ pair_keys,
                                              uint32_t* __restrict__ pair_vals, uint32_t pair_cap, int tiles_x,
                                              uint2* __restrict__ ranges, uint32_t tiles, uint32_t spin_limit) {
-    __shared__ uint32_t s_off[BIN_TILE];  // exclusive pair offsets of the tile's entries
+    __shared__ uint32_t s_off[BIN_TILE + 1];  // exclusive pair offsets of the tile's entries, and their sum
     __shared__ uint32_t s_slot[BIN_TILE];
     __shared__ uint32_t s_box[BIN_TILE];  // tx0 | ty0 << 16
     __shared__ uint16_t s_bw[BIN_TILE];
-    __shared__ uint32_t s_map[1024];  // emission step: entry + 1 at each entry's first pair position
+    __shared__ uint4 s_map[8][BIN_CHUNK / 4];  // [warp]: entry + 1 at each entry's first place in the chunk
     __shared__ uint32_t s_hist[HIST ? 768 : 1];
     __shared__ uint32_t s_scan[8];
     __shared__ uint32_t s_tile, s_epoch, s_base, s_draw;
-    const uint32_t tid = threadIdx.x;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
     frame_step(order, boxes, epoch_word);
     // every tile's range starts empty
     for (uint32_t i = blockIdx.x * 256u + tid; i < tiles; i += gridDim.x * 256u) ranges[i] = make_uint2(0u, 0u);
@@ -64,7 +69,7 @@ __global__ void __launch_bounds__(256, BIN_CTAS) k_bin(const uint32_t* __restric
         return;
     }
     if (tile == 0 && tid == 0) fc->draw = draw;
-    // per-entry tile counts (4 consecutive entries per thread keep the thread order = depth order)
+    // per-entry tile counts (consecutive entries per thread keep the thread order = depth order)
     uint32_t cnt[BIN_PER], tsum = 0;
 #pragma unroll
     for (int e = 0; e < BIN_PER; ++e) {
@@ -96,6 +101,7 @@ __global__ void __launch_bounds__(256, BIN_CTAS) k_bin(const uint32_t* __restric
         s_off[tid * BIN_PER + e] = off;
         off += cnt[e];
     }
+    if (tid == 255u) s_off[BIN_TILE] = off;
     if (tid < 32) {
         if (tid == 0) lb_store(status + lb_word(tile), lb_pack(epoch, tile == 0 ? LB_INC : LB_AGG, btot));
         const uint32_t excl = lookback_single<BIN_LB>(status, tile, epoch, spin_limit, &fc->err);
@@ -110,76 +116,63 @@ __global__ void __launch_bounds__(256, BIN_CTAS) k_bin(const uint32_t* __restric
     }
     __syncthreads();
     const uint32_t gbase = s_base;
-    // Load-balanced emission, 1024 pairs per step: pair q of this CTA belongs to the last entry whose
-    // offset is <= q.  Each entry with pairs marks its first pair's position (entry + 1), and an
-    // inclusive max-scan over the step's positions (carrying the previous step's last entry) hands
-    // every position its entry; thread t emits positions 4t .. 4t + 3.
-    uint32_t carry = 0u;
-    for (uint32_t q0 = 0; q0 < btot; q0 += 1024u) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) s_map[tid * 4 + k] = 0u;
-        __syncthreads();
-#pragma unroll
-        for (int e = 0; e < BIN_PER; ++e) {
-            const uint32_t ei = tid * (uint32_t)BIN_PER + e;
-            const uint32_t o = s_off[ei];
-            if (cnt[e] != 0u && o >= q0 && o - q0 < 1024u) s_map[o - q0] = ei + 1u;
+    // Emission in chunks of 128 pairs, dealt to the warps in turn (the nearest splats, first in the order, may
+    // cover thousands of tiles each), no CTA barriers: the warp finds the entry of the chunk's first pair by two
+    // ballots over the offsets, entries that start in the chunk mark their first place (entry + 1), and the last mark
+    // at or before a place is its entry.  Lanes emit consecutive pairs.
+    uint32_t* map = reinterpret_cast<uint32_t*>(s_map[w]);
+    const uint32_t le = 0xFFFFFFFFu >> (31u - lane);
+    for (uint32_t q0 = w * BIN_CHUNK; q0 < btot; q0 += 8u * BIN_CHUNK) {
+        s_map[w][lane] = make_uint4(0u, 0u, 0u, 0u);
+        // the last entry that starts at or before q0 (offsets rise; the first one is 0): a 32nd of the tile, then entry
+        constexpr uint32_t B = BIN_TILE / 32;
+        const uint32_t blk = (uint32_t)__popc(__ballot_sync(FULL_MASK, s_off[B * lane] <= q0)) - 1u;
+        uint32_t first = B * blk + (uint32_t)__popc(__ballot_sync(FULL_MASK, lane < B && s_off[B * blk + lane] <= q0)) - 1u;
+        const uint32_t before = first + 1u;  // as a mark
+        __syncwarp();
+        for (bool more = true; more; first += 32u) {
+            const uint32_t e = first + 1u + lane;
+            const uint32_t o = e < (uint32_t)BIN_TILE ? s_off[e] : btot;
+            if (o < q0 + BIN_CHUNK && o < btot && s_off[e + 1u] != o) map[o - q0] = e + 1u;
+            more = __all_sync(FULL_MASK, o < q0 + BIN_CHUNK && o < btot);
         }
-        __syncthreads();
-        uint32_t v[4], m = carry;
+        __syncwarp();
+        uint32_t carry = before;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            m = max(m, s_map[tid * 4 + k]);
-            v[k] = m;  // thread-local inclusive max (with the carry)
-        }
-        uint32_t x = m;  // inclusive max-scan of the thread maxima over the warp
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(FULL_MASK, x, o);
-            if ((tid & 31u) >= (uint32_t)o) x = max(x, y);
-        }
-        const uint32_t before_in_warp = __shfl_up_sync(FULL_MASK, x, 1);
-        if ((tid & 31u) == 31u) s_scan[tid >> 5] = x;
-        __syncthreads();
-        uint32_t before = (tid & 31u) ? before_in_warp : 0u, all = 0u;
-#pragma unroll
-        for (uint32_t wi = 0; wi < 8; ++wi) {
-            const uint32_t sw = s_scan[wi];
-            before = wi < (tid >> 5) ? max(before, sw) : before;
-            all = max(all, sw);
-        }
-        carry = all;  // the entry at the step's last position: the carry into the next step
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t q = q0 + tid * 4u + k;
-            const uint32_t marked = max(before, v[k]);  // >= 1: position 0 of the first step is marked
-            if (q >= btot || marked == 0u) break;
-            const uint32_t e = marked - 1u;
-            const uint32_t li = q - s_off[e];
-            const uint32_t bw = s_bw[e], box = s_box[e];
-            // li / bw and li % bw (li < 2^24): float estimate, corrected by one step
-            uint32_t dy = __float2uint_rz(__fdividef((float)li, (float)bw));
-            int32_t dx = (int32_t)(li - dy * bw);
-            if (dx < 0) {
-                --dy;
-                dx += (int32_t)bw;
-            } else if (dx >= (int32_t)bw) {
-                ++dy;
-                dx -= (int32_t)bw;
-            }
-            const uint32_t tid_tile = ((box >> 16) + dy) * (uint32_t)tiles_x + (box & 0xFFFFu) + (uint32_t)dx;
-            const uint32_t g = gbase + q;
-            if (g < pair_cap) {
-                pair_keys[g] = tid_tile;
-                pair_vals[g] = s_slot[e];
-                if (HIST) {
-                    atomicAdd(&s_hist[tid_tile & 255u], 1u);
-                    atomicAdd(&s_hist[256u + ((tid_tile >> 8) & 255u)], 1u);
-                    atomicAdd(&s_hist[512u + ((tid_tile >> 16) & 255u)], 1u);
+        for (uint32_t k = 0; k < BIN_CHUNK; k += 32u) {
+            const uint32_t q = q0 + k + lane;
+            const uint32_t mark = map[k + lane];
+            const uint32_t upto = __ballot_sync(FULL_MASK, mark != 0u) & le;
+            const uint32_t found = __shfl_sync(FULL_MASK, mark, upto ? 31 - __clz(upto) : 0);
+            const uint32_t e = (upto ? found : carry) - 1u;
+            carry = __shfl_sync(FULL_MASK, e, 31) + 1u;
+            if (q < btot) {
+                const uint32_t li = q - s_off[e];
+                const uint32_t bw = s_bw[e], box = s_box[e];
+                // li / bw and li % bw (li < 2^24): float estimate, corrected by one step
+                uint32_t dy = __float2uint_rz(__fdividef((float)li, (float)bw));
+                int32_t dx = (int32_t)(li - dy * bw);
+                if (dx < 0) {
+                    --dy;
+                    dx += (int32_t)bw;
+                } else if (dx >= (int32_t)bw) {
+                    ++dy;
+                    dx -= (int32_t)bw;
+                }
+                const uint32_t tid_tile = ((box >> 16) + dy) * (uint32_t)tiles_x + (box & 0xFFFFu) + (uint32_t)dx;
+                const uint32_t g = gbase + q;
+                if (g < pair_cap) {
+                    pair_keys[g] = tid_tile;
+                    pair_vals[g] = s_slot[e];
+                    if (HIST) {
+                        atomicAdd(&s_hist[tid_tile & 255u], 1u);
+                        atomicAdd(&s_hist[256u + ((tid_tile >> 8) & 255u)], 1u);
+                        atomicAdd(&s_hist[512u + ((tid_tile >> 16) & 255u)], 1u);
+                    }
                 }
             }
         }
-        __syncthreads();  // s_map and s_scan are rewritten by the next step
+        __syncwarp();
     }
     if (HIST) {
         __syncthreads();

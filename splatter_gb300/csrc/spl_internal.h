@@ -79,7 +79,7 @@ struct spl_renderer {
     float4* rec = nullptr;
     uint2* boxes = nullptr;  // pixel box of each record, for the binning kernel
     uint64_t* st_cull = nullptr;  // [LB_LINE * ceil(max_n/1024)]
-    uint64_t* st_bin = nullptr;   // [LB_LINE * ceil(max_n/1024)]
+    uint64_t* st_bin = nullptr;   // [LB_LINE * ceil(max_n/512)]
     uint32_t *pk_a = nullptr, *pk_b = nullptr, *pv_a = nullptr, *pv_b = nullptr;
     FrameCounters* fc = nullptr;
     FrameCounters* fc_sort = nullptr;  // counters of spl_sort_pairs

@@ -63,7 +63,7 @@ constexpr int CULL_TILE_SMALL = 1024;  // the same in frames of at most CULL_SMA
 constexpr uint32_t CULL_SMALL_MAX = 1u << 19;
 constexpr int SORT_TILE = 4096;        // keys per onesweep tile (256 threads x 16)
 constexpr size_t LB_LINE = 16;          // look-back status: words between one tile's and the next (128 bytes)
-constexpr int BIN_TILE = 1024;         // draw entries per binning tile (256 threads x 4)
+constexpr int BIN_TILE = 512;          // draw entries per binning tile (256 threads x 2)
 constexpr float FP32_T_MIN = 1e-4f;    // fp32 blend mode stops a pixel below this transmittance
 
 struct SceneView {
