@@ -515,7 +515,7 @@ int spl_renderer_launches_per_frame(const spl_renderer* r, uint32_t width, uint3
     // frame_begin, cull, preprocess, depth sort (one cooperative launch or 4 onesweep passes),
     // bin, pair sort (one cooperative launch or one launch per pass), ranges, tile
     // order, raster
-    return 1 + 1 + 1 + depth_sort + 1 + (coop ? 1 : pair_passes) + 1 + (r->order_tiles ? 1 : 0) + 1;
+    return 1 + 1 + 1 + depth_sort + 1 + (coop ? 1 : pair_passes) + 1 + (r->order_tiles && raster_orders_tiles(tiles) ? 1 : 0) + 1;
 }
 
 static int render_backward(spl_renderer* r, const spl_scene* scene, const float* image_device,

@@ -65,7 +65,7 @@ __device__ __forceinline__ uint32_t reduce10_over4(const float* g, uint32_t li, 
 // of three, more atomics) 116 us; lists as record indices instead of bit words 111 us.
 template <bool RECT, bool FAR>
 __global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restrict__ ranges,
-                                                         const uint32_t* __restrict__ tile_order,
+                                                         const uint4* __restrict__ tile_order,
                                                          const uint32_t* __restrict__ pair_vals,
                                                          const float4* __restrict__ rec, int W, int H, int tiles_x,
                                                          float margin, float psx, float psy,
@@ -80,14 +80,15 @@ __global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restr
     const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5, lt = lanemask_lt();
     const uint32_t grp = lane >> 2, li = lane & 3u;
     // the forward's most-pairs-first order of this frame's tiles, when it made one
-    const int tile = tile_order ? (int)__ldg(tile_order + blockIdx.x) : (int)blockIdx.x;
+    uint2 rg;
+    int tile;
+    ordered_tile(ranges, tile_order, rg, tile);
     const int tx = tile % tiles_x, ty = tile / tiles_x;
     const int wx0 = tx * TILE_PIXELS, ty0 = ty * TILE_PIXELS;
     const uint32_t col = 2u * grp + (li & 1u), row = li >> 1;
     const int px = wx0 + (int)col, py = ty0 + 2 * (int)w + (int)row;
     const float X = (float)px + 0.5f, Y = (float)py + 0.5f;
     const uint32_t my_pixel = 1u << (16u * row + col);  // in a strip's row mask
-    const uint2 rg = ranges[tile];
     const bool inside = px < W && py < H;
     float Cf[3] = {0.0f, 0.0f, 0.0f}, gC[3] = {0.0f, 0.0f, 0.0f}, Tf = 1.0f, gT = 0.0f;
     if (inside) {
@@ -373,7 +374,7 @@ __global__ void __launch_bounds__(128) k_preprocess_backward_double(SceneView s,
 
 void launch_backward(int sh_order, bool covariance, bool rect, const SceneView& s, const Uniforms& u,
                      const uint32_t* idx, const FrameCounters* fc, const uint2* boxes, const uint2* ranges,
-                     const uint32_t* tile_order, const uint32_t* pair_vals, const float4* rec, const float4* image,
+                     const uint4* tile_order, const uint32_t* pair_vals, const float4* rec, const float4* image,
                      const float4* grad_image, float* grad_rec, uint32_t* deferred,
                      uint32_t max_n, float* gx, float* gy, float* gz, float4* grot, float4* gscale_alpha, float* gsh,
                      bool accumulate, cudaStream_t st) {
@@ -386,6 +387,7 @@ void launch_backward(int sh_order, bool covariance, bool rect, const SceneView& 
     if (zg == 0) zg = 1;
     k_zero_grad_rec<<<zg, 256, 0, st>>>(grad_rec, fc, deferred);
     const int grid = tiles_x * tiles_y;
+    if (!raster_orders_tiles((uint64_t)grid)) tile_order = nullptr;
     if (grid > 0) {
         auto k = !rect ? k_raster_backward<false, true>
                        : (fabsf(u.margin) <= RASTER_NEAR_MARGIN ? k_raster_backward<true, false> : k_raster_backward<true, true>);

@@ -92,7 +92,7 @@ struct spl_renderer {
     uint64_t* st_pairs = nullptr;      // onesweep mode: look-back status of the <= 3 pair passes
     FrameCounters* host_fc = nullptr;  // pinned
     uint2* ranges = nullptr;
-    uint32_t* tile_order = nullptr;  // the raster's tile order, most pairs first (ranges_cap entries)
+    uint4* tile_order = nullptr;     // the raster's tile order, most pairs first (ranges_cap entries)
     bool order_tiles = true;         // off where concurrent frames already hide the raster's tail (serving)
     // render_frame replays a frame graph it captured itself once a viewport and scene size repeat
     bool frame_graphs = true;

@@ -7,6 +7,7 @@ namespace spl {
 
 constexpr int RASTER_BATCH = 256;
 constexpr int RASTER_WORDS = RASTER_BATCH / 32;
+constexpr uint32_t RASTER_CTAS = 6;  // of k_raster per SM
 constexpr float RASTER_NEAR_MARGIN = 9.0f;  // up to this margin a covered pixel's exponent stays above -87
 
 // Two float operations per instruction on packed pairs (the results of the scalar operations, each rounded
@@ -34,6 +35,18 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
         : "=f"(d.x), "=f"(d.y)
         : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
     return d;
+}
+
+// The CTA's tile and its pair range: the next entry of the tile order, or row-major without one.
+__device__ __forceinline__ void ordered_tile(const uint2* ranges, const uint4* tile_order, uint2& range, int& tile) {
+    if (tile_order) {
+        const uint4 e = __ldg(tile_order + blockIdx.x);
+        range = make_uint2(e.x, e.y);
+        tile = (int)e.z;
+    } else {
+        range = __ldg(ranges + blockIdx.x);
+        tile = (int)blockIdx.x;
+    }
 }
 
 // Highest set bit of x (x != 0).

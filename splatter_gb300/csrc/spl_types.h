@@ -110,9 +110,10 @@ void launch_bin(int mode, bool hist, const uint32_t* order, const uint2* boxes, 
                 cudaStream_t st);
 void launch_tile_ranges(const uint32_t* pair_keys, const FrameCounters* fc, uint32_t pair_cap, uint2* ranges,
                         cudaStream_t st);
-// Orders the tiles most pairs first (tile_order, one entry per tile), then rasterises them in that order;
-// with tile_order == nullptr in row-major order.
-void launch_raster(bool rect, int blend, const uint2* ranges, uint32_t* tile_order, const uint32_t* pair_vals,
+bool raster_orders_tiles(uint64_t tiles);  // whether viewports of that many tiles are rasterised in order
+// Orders the tiles most pairs first (tile_order, one entry per tile; only where raster_orders_tiles), then rasterises them in that order;
+// with tile_order == nullptr in row-major order.  Entries: (pair range, tile, -).
+void launch_raster(bool rect, int blend, const uint2* ranges, uint4* tile_order, const uint32_t* pair_vals,
                    const float4* rec, const Uniforms& u, void* out, cudaStream_t st);
 void launch_load_records(const float* records62, uint32_t count, float* x, float* y, float* z, float4* rot,
                          float4* scale_alpha, float* sh, cudaStream_t st);
@@ -149,7 +150,7 @@ void launch_l2_loss_backward(const float* image, const float* target, uint64_t p
 // needles and discs whose vertex-stage sweep runs in double).
 void launch_backward(int sh_order, bool covariance, bool rect, const SceneView& s, const Uniforms& u,
                      const uint32_t* idx, const FrameCounters* fc, const uint2* boxes, const uint2* ranges,
-                     const uint32_t* tile_order, const uint32_t* pair_vals, const float4* rec, const float4* image,
+                     const uint4* tile_order, const uint32_t* pair_vals, const float4* rec, const float4* image,
                      const float4* grad_image,
                      float* grad_rec, uint32_t* deferred,
                      uint32_t max_n, float* gx, float* gy, float* gz, float4* grot, float4* gscale_alpha, float* gsh,

@@ -51,3 +51,24 @@ def test_lists_equal_the_oracle(cuda, n, size, margin, rects):
         assert got.dtype == ref.dtype and got.tobytes() == ref.tobytes(), (blend, np.argwhere(got != ref)[:4].tolist())
         s.close()
         r.close()
+
+
+@pytest.mark.parametrize("size", [(608, 384), (1328, 176), (1024, 1024), (272, 3856)])
+def test_tile_order_covers_the_viewport(cuda, size):
+    """Viewports at the edges of the tile order: 912 tiles (all resident, no order) and 913, one 4096-tile step
+    and one tile more."""
+    import torch
+    n, (w, h) = 4000, size
+    rec = stack_of_splats(n, seed=3)
+    rec[:, 0:3] *= 4.0
+    config = Configuration(max_splat_count=n, spherical_harmonics_order=1, field_of_view_y=math.radians(70))
+    cam = default_cam(dist=4.0)
+    r = Renderer(config)
+    s = Scene(r, n)
+    s.load_chunk(rec)
+    img = r.render_frame(s, cam, w, h, out=torch.full((h, w, 4), 7, dtype=torch.uint8, device="cuda"))
+    torch.cuda.synchronize()
+    ref, _ = oracle.render(oracle_uniforms(oracle, config, cam, w, h), oracle_cfg(oracle, config), oracle.load_transform(rec))
+    assert np.array_equal(img.cpu().numpy(), ref)
+    s.close()
+    r.close()
