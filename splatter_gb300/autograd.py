@@ -24,20 +24,41 @@ from .renderer import BlendMode, Renderer, _stream_ptr
 __all__ = ["render_splats", "render_raw", "render_raw_views", "activate", "activate_native", "l2_image_loss"]
 
 
+# A pass over a small scene is bound by the host: a view, an allocation or a launch of torch costs 5 to 20 us there,
+# about what a kernel of this library takes on 20k splats.  So the arrays that only this library sees are parts of
+# one tensor, addressed by their offsets, and the stream is looked up once a pass (a step of fitting 20k splats at
+# 256x192: 641 us with a tensor per array, 581 us so).
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+def _planes(t, n):
+    """The addresses of a contiguous (3, n) float32 tensor's rows."""
+    p = t.data_ptr()
+    return p, p + 4 * n, p + 8 * n
+
+
+class _Splats:
+    """n activated splats, or their gradients, in one tensor of 11 n floats: rotation (n, 4), scale and opacity
+    (n, 4), centre planes (3, n).  Every part starts on a 16-byte boundary."""
+
+    def __init__(self, data, n):
+        self.data, self.n = data, n
+        self.rot = data.data_ptr()
+        self.scale_alpha = self.rot + 16 * n
+        x = self.rot + 32 * n
+        self.planes = (x, x + 4 * n, x + 8 * n)
 
 
 class _WrappedScene:
-    """A scene over caller-owned device tensors (spl_scene_wrap); keeps the tensors alive."""
+    """A scene over device arrays (spl_scene_wrap): n splats whose x, y, z, rotation, scale_alpha and sh start at
+    the addresses given.  Keeps the tensors in `keep`, which hold the arrays, alive."""
 
-    def __init__(self, renderer, xyz, rot, scale_alpha, sh):
+    def __init__(self, renderer, n, planes, rot, scale_alpha, sh, keep):
         self._lib = _lib.load()
-        self._keep = (xyz, rot, scale_alpha, sh)
-        n = rot.shape[0]
+        self._keep = keep
         h = ctypes.c_void_p()
-        check(self._lib.spl_scene_wrap(renderer.handle, n, _ptr(xyz[0]), _ptr(xyz[1]), _ptr(xyz[2]), _ptr(rot),
-                                       _ptr(scale_alpha), _ptr(sh), ctypes.byref(h)))
+        check(self._lib.spl_scene_wrap(renderer.handle, n, *planes, rot, scale_alpha, sh, ctypes.byref(h)))
         self._h = h
 
     @property
@@ -76,7 +97,9 @@ class _RenderSplats:  # built lazily so that importing the package does not impo
                     rot = rot.contiguous()
                     scale_alpha = scale_alpha.contiguous()
                     sh = sh.contiguous()
-                    scene = _WrappedScene(renderer, xyz, rot, scale_alpha, sh)
+                    n = rot.shape[0]
+                    scene = _WrappedScene(renderer, n, _planes(xyz, n), _ptr(rot), _ptr(scale_alpha), _ptr(sh),
+                                          (xyz, rot, scale_alpha, sh))
                     img = renderer.render_frame(scene, camera_to_world, width, height)
                     ctx.renderer = renderer
                     ctx.scene = scene
@@ -97,8 +120,8 @@ class _RenderSplats:  # built lazily so that importing the package does not impo
                     gsa = torch.zeros_like(sa)
                     gsh = torch.zeros_like(sh)
                     g = grad_img.contiguous().float()
-                    check(r._lib.spl_render_backward(r.handle, ctx.scene.handle, _ptr(img), _ptr(g), _ptr(gxyz[0]),
-                                                     _ptr(gxyz[1]), _ptr(gxyz[2]), _ptr(grot), _ptr(gsa), _ptr(gsh),
+                    check(r._lib.spl_render_backward(r.handle, ctx.scene.handle, _ptr(img), _ptr(g),
+                                                     *_planes(gxyz, rot.shape[0]), _ptr(grot), _ptr(gsa), _ptr(gsh),
                                                      _stream_ptr(None)))
                     return gxyz, grot, gsa, gsh, None, None, None, None
 
@@ -120,6 +143,27 @@ def _frame_ready(ctx):
     _ensure_frame(ctx.renderer, ctx.scene, ctx.cam, *ctx.size)
 
 
+def _activated_scene(torch, means, quats, log_scales, logits, sh, stream):
+    """Activates the parameters (contiguous) on `stream`; returns wrap(renderer), the scene of the result."""
+    n = quats.shape[0]
+    splats = _Splats(torch.empty(11 * n, device=quats.device, dtype=torch.float32), n)
+    check(_lib.load().spl_activate_splats(n, _ptr(means), _ptr(quats), _ptr(log_scales), _ptr(logits), *splats.planes,
+                                          splats.rot, splats.scale_alpha, stream.cuda_stream))
+    return lambda r: _WrappedScene(r, n, splats.planes, splats.rot, splats.scale_alpha, _ptr(sh), (splats, sh))
+
+
+def _activation_grads(torch, quats, log_scales, splats, grads, st):
+    """The gradients of means, quaternions, log-scales and logits from those of the activated splats."""
+    n = splats.n
+    f32 = dict(device=quats.device, dtype=torch.float32)
+    g_means, g_quats = torch.empty((n, 3), **f32), torch.empty((n, 4), **f32)
+    g_logs, g_logits = torch.empty((n, 3), **f32), torch.empty((n,), **f32)
+    check(_lib.load().spl_activate_splats_backward(n, _ptr(quats), _ptr(log_scales), splats.rot, splats.scale_alpha,
+                                                   *grads.planes, grads.rot, grads.scale_alpha, _ptr(g_means),
+                                                   _ptr(g_quats), _ptr(g_logs), _ptr(g_logits), st))
+    return g_means, g_quats, g_logs, g_logits
+
+
 class _RenderRaw:  # built lazily, like _RenderSplats
     fn = None
 
@@ -133,17 +177,9 @@ class _RenderRaw:  # built lazily, like _RenderSplats
                 def forward(ctx, means, quats, log_scales, logits, sh, renderer, camera_to_world, width, height):
                     means, quats, log_scales, logits, sh = (t.contiguous() for t in (means, quats, log_scales, logits,
                                                                                       sh))
-                    n = quats.shape[0]
-                    f32 = dict(device=quats.device, dtype=torch.float32)
-                    xyz = torch.empty((3, n), **f32)
-                    rot = torch.empty((n, 4), **f32)
-                    sa = torch.empty((n, 4), **f32)
-                    lib = _lib.load()
-                    check(lib.spl_activate_splats(n, _ptr(means), _ptr(quats), _ptr(log_scales), _ptr(logits),
-                                                  _ptr(xyz[0]), _ptr(xyz[1]), _ptr(xyz[2]), _ptr(rot), _ptr(sa),
-                                                  _stream_ptr(None)))
-                    scene = _WrappedScene(renderer, xyz, rot, sa, sh)
-                    img = renderer.render_frame(scene, camera_to_world, width, height)
+                    st = torch.cuda.current_stream()
+                    scene = _activated_scene(torch, means, quats, log_scales, logits, sh, st)(renderer)
+                    img = renderer.render_frame(scene, camera_to_world, width, height, stream=st)
                     ctx.renderer = renderer
                     ctx.scene = scene
                     ctx.cam = np.ascontiguousarray(np.asarray(camera_to_world, np.float32).reshape(16))
@@ -157,26 +193,14 @@ class _RenderRaw:  # built lazily, like _RenderSplats
                     img, quats, log_scales = ctx.saved_tensors
                     _frame_ready(ctx)
                     r = ctx.renderer
-                    xyz, rot, sa, sh = ctx.scene._keep
-                    n = rot.shape[0]
-                    gxyz = torch.zeros_like(xyz)
-                    grot = torch.zeros_like(rot)
-                    gsa = torch.zeros_like(sa)
+                    splats, sh = ctx.scene._keep
+                    grads = _Splats(torch.zeros_like(splats.data), splats.n)
                     gsh = torch.zeros_like(sh)
                     g = grad_img.contiguous().float()
                     st = _stream_ptr(None)
-                    check(r._lib.spl_render_backward(r.handle, ctx.scene.handle, _ptr(img), _ptr(g), _ptr(gxyz[0]),
-                                                     _ptr(gxyz[1]), _ptr(gxyz[2]), _ptr(grot), _ptr(gsa), _ptr(gsh),
-                                                     st))
-                    g_means = torch.empty((n, 3), device=rot.device, dtype=torch.float32)
-                    g_quats = torch.empty((n, 4), device=rot.device, dtype=torch.float32)
-                    g_logs = torch.empty((n, 3), device=rot.device, dtype=torch.float32)
-                    g_logits = torch.empty((n,), device=rot.device, dtype=torch.float32)
-                    check(r._lib.spl_activate_splats_backward(n, _ptr(quats), _ptr(log_scales), _ptr(rot), _ptr(sa),
-                                                              _ptr(gxyz[0]), _ptr(gxyz[1]), _ptr(gxyz[2]),
-                                                              _ptr(grot), _ptr(gsa), _ptr(g_means), _ptr(g_quats),
-                                                              _ptr(g_logs), _ptr(g_logits), st))
-                    return g_means, g_quats, g_logs, g_logits, gsh, None, None, None, None
+                    check(r._lib.spl_render_backward(r.handle, ctx.scene.handle, _ptr(img), _ptr(g), *grads.planes,
+                                                     grads.rot, grads.scale_alpha, _ptr(gsh), st))
+                    return *_activation_grads(torch, quats, log_scales, splats, grads, st), gsh, None, None, None, None
 
             cls.fn = RenderRaw
         return cls.fn
@@ -195,24 +219,17 @@ class _RenderRawViews:  # built lazily, like _RenderSplats
                 def forward(ctx, means, quats, log_scales, logits, sh, renderers, cameras, width, height):
                     means, quats, log_scales, logits, sh = (t.contiguous() for t in (means, quats, log_scales, logits,
                                                                                       sh))
-                    n = quats.shape[0]
-                    f32 = dict(device=quats.device, dtype=torch.float32)
-                    xyz = torch.empty((3, n), **f32)
-                    rot = torch.empty((n, 4), **f32)
-                    sa = torch.empty((n, 4), **f32)
-                    lib = _lib.load()
-                    check(lib.spl_activate_splats(n, _ptr(means), _ptr(quats), _ptr(log_scales), _ptr(logits),
-                                                  _ptr(xyz[0]), _ptr(xyz[1]), _ptr(xyz[2]), _ptr(rot), _ptr(sa),
-                                                  _stream_ptr(None)))
-                    out = torch.empty((len(cameras), height, width, 4), **f32)
+                    st = torch.cuda.current_stream()
+                    wrap = _activated_scene(torch, means, quats, log_scales, logits, sh, st)
+                    out = torch.empty((len(cameras), height, width, 4), device=quats.device, dtype=torch.float32)
                     scenes, views = {}, []
                     for v, cam in enumerate(cameras):
                         r = renderers[v % len(renderers)]
                         if id(r) not in scenes:
-                            scenes[id(r)] = _WrappedScene(r, xyz, rot, sa, sh)
+                            scenes[id(r)] = wrap(r)
                         scene = scenes[id(r)]
                         c = np.ascontiguousarray(np.asarray(cam, np.float32).reshape(16))
-                        r.render_frame(scene, c, width, height, out=out[v])
+                        r.render_frame(scene, c, width, height, out=out[v], stream=st)
                         r._last_frame_key = (id(scene), c.tobytes(), width, height)
                         views.append((r, scene, c))
                     ctx.views = views
@@ -224,30 +241,18 @@ class _RenderRawViews:  # built lazily, like _RenderSplats
                 def backward(ctx, grad_out):
                     out, quats, log_scales = ctx.saved_tensors
                     w, h = ctx.size
-                    xyz, rot, sa, sh = ctx.views[0][1]._keep
-                    n = rot.shape[0]
-                    gxyz = torch.zeros_like(xyz)
-                    grot = torch.zeros_like(rot)
-                    gsa = torch.zeros_like(sa)
+                    splats, sh = ctx.views[0][1]._keep
+                    grads = _Splats(torch.zeros_like(splats.data), splats.n)
                     gsh = torch.zeros_like(sh)
                     g = grad_out.contiguous().float()
                     st = _stream_ptr(None)
                     # the views in order, each adding its gradients in place
                     for v, (r, scene, c) in enumerate(ctx.views):
                         _ensure_frame(r, scene, c, w, h)
-                        check(r._lib.spl_render_backward_accumulate(r.handle, scene.handle, _ptr(out[v]), _ptr(g[v]),
-                                                                    _ptr(gxyz[0]), _ptr(gxyz[1]), _ptr(gxyz[2]),
-                                                                    _ptr(grot), _ptr(gsa), _ptr(gsh), st))
-                    g_means = torch.empty((n, 3), device=rot.device, dtype=torch.float32)
-                    g_quats = torch.empty((n, 4), device=rot.device, dtype=torch.float32)
-                    g_logs = torch.empty((n, 3), device=rot.device, dtype=torch.float32)
-                    g_logits = torch.empty((n,), device=rot.device, dtype=torch.float32)
-                    check(_lib.load().spl_activate_splats_backward(n, _ptr(quats), _ptr(log_scales), _ptr(rot),
-                                                                   _ptr(sa), _ptr(gxyz[0]), _ptr(gxyz[1]),
-                                                                   _ptr(gxyz[2]), _ptr(grot), _ptr(gsa),
-                                                                   _ptr(g_means), _ptr(g_quats), _ptr(g_logs),
-                                                                   _ptr(g_logits), st))
-                    return g_means, g_quats, g_logs, g_logits, gsh, None, None, None, None
+                        check(r._lib.spl_render_backward_accumulate(
+                            r.handle, scene.handle, _ptr(out) + 4 * out.stride(0) * v, _ptr(g) + 4 * g.stride(0) * v,
+                            *grads.planes, grads.rot, grads.scale_alpha, _ptr(gsh), st))
+                    return *_activation_grads(torch, quats, log_scales, splats, grads, st), gsh, None, None, None, None
 
             cls.fn = RenderRawViews
         return cls.fn
@@ -271,7 +276,7 @@ def activate_native(means, quats, log_scales, opacity_logits):
     f32 = dict(device=quats.device, dtype=torch.float32)
     xyz, rot, sa = torch.empty((3, n), **f32), torch.empty((n, 4), **f32), torch.empty((n, 4), **f32)
     check(_lib.load().spl_activate_splats(n, _ptr(means), _ptr(quats), _ptr(log_scales), _ptr(opacity_logits),
-                                          _ptr(xyz[0]), _ptr(xyz[1]), _ptr(xyz[2]), _ptr(rot), _ptr(sa),
+                                          *_planes(xyz, n), _ptr(rot), _ptr(sa),
                                           _stream_ptr(None)))
     return xyz, rot, sa
 
