@@ -340,8 +340,9 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
     if (mode != DS_NONE && N > 0) {
         // four stable 8-bit passes a -> b -> a -> b -> a; pass 0 takes the compaction slot as the value
         if (coop) {
-            CU(launch_sort_coop(r->keys_a, r->keys_b, r->vals_a, r->vals_b, true, &r->fc->visible, N, 4, 0,
-                                r->coop_table, r->epoch, &r->fc->barrier[0].v, sl, &r->fc->err, st));
+            const SortBuffers io{r->keys_a, nullptr, {r->keys_a, r->keys_b}, {r->vals_a, r->vals_b}, r->keys_a, r->vals_a};
+            CU(launch_sort_coop(io, &r->fc->visible, N, 4, 0, r->coop_table, r->epoch, &r->fc->barrier[0].v, sl,
+                                &r->fc->err, st));
         } else {
             // digit histograms from the cull kernel; one launch per pass
             uint32_t *src_k = r->keys_a, *dst_k = r->keys_b, *dst_v = r->vals_b;
@@ -368,8 +369,10 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
     // stable sort of the pairs by tile id keeps each tile's list in depth order
     const int passes = tiles <= 256 ? 1 : (tiles <= 65536 ? 2 : 3);
     if (coop) {
-        CU(launch_sort_coop(r->pk_a, r->pk_b, r->pv_a, r->pv_b, false, &r->fc->pairs, (uint32_t)r->pair_cap, passes,
-                            0, r->coop_table + sort_coop_table_words(), r->epoch, &r->fc->barrier[1].v, sl, &r->fc->err, st));
+        const SortBuffers io{r->pk_a, r->pv_a, {r->pk_a, r->pk_b}, {r->pv_a, r->pv_b}, (passes & 1) ? r->pk_b : r->pk_a,
+                             (passes & 1) ? r->pv_b : r->pv_a};
+        CU(launch_sort_coop(io, &r->fc->pairs, (uint32_t)r->pair_cap, passes, 0, r->coop_table + sort_coop_table_words(),
+                            r->epoch, &r->fc->barrier[1].v, sl, &r->fc->err, st));
     } else {
         // tile-id histograms from the binning kernel
         uint32_t *ak = r->pk_a, *av = r->pv_a, *bk = r->pk_b, *bv = r->pv_b;
@@ -614,6 +617,43 @@ int spl_renderer_copy_records(spl_renderer* r, float* records_device, uint64_t c
     return SPL_OK;
 }
 
+static bool overlap(const void* a, const void* b, uint64_t bytes) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + bytes && y < x + bytes;
+}
+
+// Whether a kernel may read or write `bytes` bytes of both arrays: aligned, on the current device, and inside one
+// allocation as far as the driver says (the check that a copy makes).
+static bool sortable(const void* const (&array)[2], uint64_t bytes, unsigned align0, unsigned align1) {
+    typedef int (*AddressRange)(unsigned long long*, size_t*, unsigned long long);
+    static const AddressRange range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<AddressRange>(f);
+    }();
+    int dev = -1;
+    if (!range || cudaGetDevice(&dev) != cudaSuccess) return false;
+    for (int i = 0; i < 2; ++i) {
+        const uintptr_t p = reinterpret_cast<uintptr_t>(array[i]);
+        if (p % (i == 0 ? align0 : align1)) return false;
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, array[i]) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        unsigned long long base = 0;
+        size_t size = 0;
+        if (at.type != cudaMemoryTypeDevice || at.device != dev || range(&base, &size, p) != 0) return false;
+        if (p + bytes > base + size) return false;
+    }
+    return true;
+}
+
 int spl_sort_pairs(spl_renderer* r, const uint32_t* keys_in, const uint32_t* values_in, uint32_t* keys_out,
                    uint32_t* values_out, uint64_t count, uint32_t key_bits, void* stream) {
     if (!r || !keys_in || !values_in || !keys_out || !values_out) return fail(SPL_ERR_INVALID, "NULL argument");
@@ -622,16 +662,34 @@ int spl_sort_pairs(spl_renderer* r, const uint32_t* keys_in, const uint32_t* val
     cudaStream_t st = (cudaStream_t)stream;
     if (count == 0) return SPL_OK;
     const int passes = (int)(key_bits / 8);
-    launch_frame_begin(r->fc_sort, r->epoch, st);
-    launch_set_count(&r->fc_sort->visible, (uint32_t)count, st);
-    CU(cudaMemcpyAsync(r->keys_a, keys_in, count * 4, cudaMemcpyDeviceToDevice, st));
-    CU(cudaMemcpyAsync(r->vals_a, values_in, count * 4, cudaMemcpyDeviceToDevice, st));
-    CU(launch_sort_coop(r->keys_a, r->keys_b, r->vals_a, r->vals_b, false, &r->fc_sort->visible, (uint32_t)count,
-                        passes, 0, r->coop_table, r->epoch, &r->fc_sort->barrier[0].v, r->spin_limit, &r->fc_sort->err, st));
-    const uint32_t* kr = (passes & 1) ? r->keys_b : r->keys_a;
-    const uint32_t* vr = (passes & 1) ? r->vals_b : r->vals_a;
-    CU(cudaMemcpyAsync(keys_out, kr, count * 4, cudaMemcpyDeviceToDevice, st));
-    CU(cudaMemcpyAsync(values_out, vr, count * 4, cudaMemcpyDeviceToDevice, st));
+    // The first pass reads the caller's input and the last writes the output.  A copy through the scratch stays
+    // where the kernel needs more than a copy does: memory that is not this device's or not wholly inside an
+    // allocation, unaligned arrays, an output that overlaps the other one, or the input of a single pass.
+    // 3.5M pairs of 32-bit keys: 117 us, 154 us with the four copies.
+    const uint64_t bytes = count * 4;
+    const void* out[2] = {keys_out, values_out};
+    const void* in[2] = {keys_in, values_in};
+    const bool write = !overlap(keys_out, values_out, bytes) && sortable(out, bytes, 4, 4);
+    bool read = sortable(in, bytes, 16, 4);
+    for (int i = 0; i < 4 && passes == 1; ++i) read = read && !overlap(in[i & 1], out[i >> 1], bytes);
+    SortBuffers io{keys_in, values_in, {r->keys_a, r->keys_b}, {r->vals_a, r->vals_b}, keys_out, values_out};
+    launch_frame_begin(r->fc_sort, r->epoch, (uint32_t)count, st);
+    if (!read) {
+        CU(cudaMemcpyAsync(r->keys_a, keys_in, bytes, cudaMemcpyDeviceToDevice, st));
+        CU(cudaMemcpyAsync(r->vals_a, values_in, bytes, cudaMemcpyDeviceToDevice, st));
+        io.keys_in = r->keys_a;
+        io.vals_in = r->vals_a;
+    }
+    if (!write) {
+        io.keys_out = io.keys[passes & 1];
+        io.vals_out = io.vals[passes & 1];
+    }
+    CU(launch_sort_coop(io, &r->fc_sort->visible, (uint32_t)count, passes, 0, r->coop_table, r->epoch,
+                        &r->fc_sort->barrier[0].v, r->spin_limit, &r->fc_sort->err, st));
+    if (!write) {
+        CU(cudaMemcpyAsync(keys_out, io.keys_out, bytes, cudaMemcpyDeviceToDevice, st));
+        CU(cudaMemcpyAsync(values_out, io.vals_out, bytes, cudaMemcpyDeviceToDevice, st));
+    }
     return SPL_OK;
 }
 

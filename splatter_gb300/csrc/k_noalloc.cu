@@ -90,8 +90,7 @@ extern "C" int spl_sort_pairs_no_alloc(const uint32_t* keys_in, const uint32_t* 
     NoAllocScratch* s = static_cast<NoAllocScratch*>(base);
     cudaStream_t st = (cudaStream_t)stream;
     const int passes = (int)(key_bits / 8);
-    launch_frame_begin(&s->fc, &s->epoch, st);  // zeroes counters, histograms and tile counters
-    launch_set_count(&s->fc.visible, (uint32_t)count, st);
+    launch_frame_begin(&s->fc, &s->epoch, (uint32_t)count, st);  // zeroes histograms and tile counters
     launch_histogram(keys_in, &s->fc.visible, (uint32_t)count, s->fc.hist_depth[0], st);
     const uint32_t* kin = keys_in;
     const uint32_t* vin = values_in;

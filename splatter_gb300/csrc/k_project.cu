@@ -29,7 +29,10 @@ __device__ __forceinline__ void counters_begin(FrameCounters* fc, uint32_t* epoc
     }
 }
 
-__global__ void k_counters_begin(FrameCounters* fc, uint32_t* epoch_word) { counters_begin(fc, epoch_word); }
+__global__ void k_counters_begin(FrameCounters* fc, uint32_t* epoch_word, uint32_t count) {
+    counters_begin(fc, epoch_word);
+    if (threadIdx.x == 0) fc->visible = count;
+}
 
 // A frame's first kernel: the counters as above, and the frame's uniform block and scene view
 // (kernel parameters here, so that a captured frame graph takes a new camera and scene by updating
@@ -45,8 +48,8 @@ __global__ void k_frame_begin(FrameCounters* fc, uint32_t* epoch_word, Uniforms 
     counters_begin(fc, epoch_word);
 }
 
-void launch_frame_begin(FrameCounters* fc, uint32_t* epoch_word, cudaStream_t st) {
-    k_counters_begin<<<1, 256, 0, st>>>(fc, epoch_word);
+void launch_frame_begin(FrameCounters* fc, uint32_t* epoch_word, uint32_t count, cudaStream_t st) {
+    k_counters_begin<<<1, 256, 0, st>>>(fc, epoch_word, count);
 }
 
 void launch_frame_begin(FrameCounters* fc, uint32_t* epoch_word, const Uniforms& u, Uniforms* d_u, const SceneView& sv,

@@ -211,8 +211,4 @@ void launch_histogram(const uint32_t* keys, const uint32_t* n_ptr, uint32_t n_ca
     k_histogram<<<grid, 256, 0, st>>>(keys, n_ptr, n_cap, hist4x256);
 }
 
-__global__ void k_set_count(uint32_t* dst, uint32_t value) { *dst = value; }
-
-void launch_set_count(uint32_t* dst, uint32_t value, cudaStream_t st) { k_set_count<<<1, 1, 0, st>>>(dst, value); }
-
 }  // namespace spl

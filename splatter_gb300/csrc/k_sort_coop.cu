@@ -432,13 +432,10 @@ __device__ __forceinline__ void long_pass(CoopSmem& sm, const CountTable& t, con
     }
 }
 
-// keys0 -> keys1 -> keys0 ... for `passes` passes starting at bit `shift0`; vals likewise (both value
-// buffers are real; with iota_first the values read by pass 0 are the input positions instead of
-// vals0).  The result of pass p is in keys1/vals1 for even p and keys0/vals0 for odd p (for at most
-// one sub-tile of keys only the last pass's buffers are written).
+// `passes` passes starting at bit `shift0` (the buffers: SortBuffers).  For at most one sub-tile of keys only the
+// last pass's buffers are written.
 __global__ void __launch_bounds__(CS_THREADS, 2)
-    k_sort_coop(uint32_t* keys0, uint32_t* keys1, uint32_t* vals0, uint32_t* vals1, int iota_first,
-                const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0, uint64_t* table,
+    k_sort_coop(SortBuffers io, const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0, uint64_t* table,
                 const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit, uint32_t* err) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CoopSmem& sm = *reinterpret_cast<CoopSmem*>(smem_raw);
@@ -460,11 +457,10 @@ __global__ void __launch_bounds__(CS_THREADS, 2)
     __syncwarp();
     if (G == 1u) {
         // n <= CS_TILE: one sub-tile.  Every pass ranks and stages it in shared memory (no count
-        // table, no grid barriers); the keys are read once and written once, to the buffers the last
-        // pass writes (keys1/vals1 after an odd number of passes, keys0/vals0 after an even one).
+        // table, no grid barriers); the keys are read once and written once.
         uint32_t key[CS_KPT], val[CS_KPT], pos[CS_KPT], first, count;
         const uint32_t wb = w * (32u * CS_KPT) + lane;
-        load_subtile<CS_KPT, false>(key, val, keys0, vals0, iota_first != 0, wb, n);
+        load_subtile<CS_KPT, false>(key, val, io.keys_in, io.vals_in, io.vals_in == nullptr, wb, n);
         for (int p = 0; p < passes; ++p) {
             rank_subtile<CS_KPT, false>(sm, key, pos, wb, n, shift0 + 8 * p, lt, first, count);
             __syncthreads();
@@ -482,15 +478,13 @@ __global__ void __launch_bounds__(CS_THREADS, 2)
                 }
             }
         }
-        uint32_t* kout = (passes & 1) ? keys1 : keys0;
-        uint32_t* vout = (passes & 1) ? vals1 : vals0;
 #pragma unroll
         for (int j = 0; j < CS_KPT; ++j) {
             const uint32_t i = tid + CS_THREADS * j;
             if (i < n) {
                 const uint2 kv = sm.buf[i];
-                kout[i] = kv.x;
-                vout[i] = kv.y;
+                io.keys_out[i] = kv.x;
+                io.vals_out[i] = kv.y;
             }
         }
         return;
@@ -498,11 +492,12 @@ __global__ void __launch_bounds__(CS_THREADS, 2)
     CountTable t{table, *epoch_word, 0u, spin_limit, err};
     const uint32_t s_begin = c * seg, s_end = min(s_begin + seg, n);
     for (int p = 0; p < passes; ++p) {
-        const uint32_t* kin = (p & 1) ? keys1 : keys0;
-        const uint32_t* vin = (p & 1) ? vals1 : vals0;
-        uint32_t* kout = (p & 1) ? keys0 : keys1;
-        uint32_t* vout = (p & 1) ? vals0 : vals1;
-        const bool iota = p == 0 && iota_first != 0;
+        const bool last = p + 1 == passes;
+        const uint32_t* kin = p == 0 ? io.keys_in : (p & 1) ? io.keys[1] : io.keys[0];
+        const uint32_t* vin = p == 0 ? io.vals_in : (p & 1) ? io.vals[1] : io.vals[0];
+        uint32_t* kout = last ? io.keys_out : (p & 1) ? io.keys[0] : io.keys[1];
+        uint32_t* vout = last ? io.vals_out : (p & 1) ? io.vals[0] : io.vals[1];
+        const bool iota = vin == nullptr;
         t.pass = (uint32_t)p;
         if (seg <= 4u * CS_THREADS)
             short_pass<4>(sm, t, kin, vin, kout, vout, iota, s_begin, s_end, n, shift0 + 8 * p, c, G, lt);
@@ -510,7 +505,7 @@ __global__ void __launch_bounds__(CS_THREADS, 2)
             short_pass<CS_KPT>(sm, t, kin, vin, kout, vout, iota, s_begin, s_end, n, shift0 + 8 * p, c, G, lt);
         else
             long_pass(sm, t, kin, vin, kout, vout, iota, s_begin, s_end, n, shift0 + 8 * p, c, G, lt);
-        if (p + 1 < passes) grid_barrier(bar, (uint32_t)(p + 1) * G, spin_limit, err);
+        if (!last) grid_barrier(bar, (uint32_t)(p + 1) * G, spin_limit, err);
     }
 }
 
@@ -531,18 +526,15 @@ int sort_coop_grid() {
 
 size_t sort_coop_table_words() { return (size_t)(CS_MAX_GRID + CS_MAX_GRID / CS_GROUP) * 256; }
 
-cudaError_t launch_sort_coop(uint32_t* keys0, uint32_t* keys1, uint32_t* vals0, uint32_t* vals1, bool iota_first,
-                             const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0, uint64_t* table,
-                             const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit, uint32_t* err,
-                             cudaStream_t st) {
+cudaError_t launch_sort_coop(const SortBuffers& io, const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0,
+                             uint64_t* table, const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit,
+                             uint32_t* err, cudaStream_t st) {
     if (n_cap == 0 || passes == 0) return cudaSuccess;
     int grid = sort_coop_grid();
     const uint32_t want = (n_cap + CS_MIN_SEG - 1) / CS_MIN_SEG;
     if ((uint32_t)grid > want) grid = (int)want;
     if (grid < 1) grid = 1;
-    int iota = iota_first ? 1 : 0;
-    void* args[] = {&keys0, &keys1, &vals0, &vals1, &iota, (void*)&n_ptr, &n_cap, &passes, &shift0, &table,
-                    (void*)&epoch_word, &bar, &spin_limit, &err};
+    void* args[] = {(void*)&io, (void*)&n_ptr, &n_cap, &passes, &shift0, &table, (void*)&epoch_word, &bar, &spin_limit, &err};
     return cudaLaunchCooperativeKernel((const void*)k_sort_coop, dim3(grid), dim3(CS_THREADS), args,
                                        sizeof(CoopSmem), st);
 }

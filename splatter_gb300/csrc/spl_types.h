@@ -80,7 +80,8 @@ struct SceneView {
 // Streaming multiprocessors of the current device (queried once per device, then cached); grids of
 // grid-stride kernels are capped at a multiple of it.
 uint32_t device_sm_count();
-void launch_frame_begin(FrameCounters* fc, uint32_t* epoch_word, cudaStream_t st);  // counters + epoch only
+// counters + epoch only, fc->visible = count (a sort outside a frame)
+void launch_frame_begin(FrameCounters* fc, uint32_t* epoch_word, uint32_t count, cudaStream_t st);
 void launch_frame_begin(FrameCounters* fc, uint32_t* epoch_word, const Uniforms& u, Uniforms* d_u, const SceneView& sv,
                         SceneView* d_sv, cudaStream_t st);
 const void* frame_begin_kernel();  // host handle of k_frame_begin (to find its node in a captured graph)
@@ -122,14 +123,21 @@ void launch_splats60_to_soa(const float* s60, uint32_t count, float* x, float* y
 void launch_soa_to_splats60(const SceneView& s, uint32_t start, uint32_t count, float* s60, cudaStream_t st);
 void launch_gather_entries(const uint32_t* keys, const uint32_t* slots, const uint32_t* idx, const FrameCounters* fc,
                            int mode, uint32_t* keys_out, uint32_t* idx_out, uint32_t cap, cudaStream_t st);
-// All passes of a stable LSD radix sort in one cooperative launch (k_sort_coop.cu).  Pass p reads
-// buffers (p even: 0, odd: 1) and writes the other.  table: sort_coop_table_words() words of its own for each
+// All passes of a stable LSD radix sort in one cooperative launch (k_sort_coop.cu).  Pass 0 reads keys_in and
+// vals_in (no vals_in: the values are the positions), the last pass writes keys_out and vals_out, and in between
+// pass p writes keys[1], vals[1] (p even) or keys[0], vals[0] (p odd) for the next.  The input may be
+// keys[0], vals[0], the output the buffer of its pass; with more than one pass the input may overlap the output.
+// keys_in is 16-byte aligned.  table: sort_coop_table_words() words of its own for each
 // sort of a frame, zero at first and never cleared (the words carry *epoch_word, never 0 and another one at
 // each launch); *bar (the grid barrier's arrival count) must be zero when the launch starts.
-cudaError_t launch_sort_coop(uint32_t* keys0, uint32_t* keys1, uint32_t* vals0, uint32_t* vals1, bool iota_first,
-                             const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0, uint64_t* table,
-                             const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit, uint32_t* err,
-                             cudaStream_t st);
+struct SortBuffers {
+    const uint32_t *keys_in, *vals_in;
+    uint32_t *keys[2], *vals[2];
+    uint32_t *keys_out, *vals_out;
+};
+cudaError_t launch_sort_coop(const SortBuffers& io, const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0,
+                             uint64_t* table, const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit,
+                             uint32_t* err, cudaStream_t st);
 size_t sort_coop_table_words();
 int sort_coop_grid();
 // The loader's activations of raw parameters and their backward (k_activate.cu).
@@ -157,7 +165,6 @@ void launch_backward(int sh_order, bool covariance, bool rect, const SceneView& 
                      bool accumulate, cudaStream_t st);
 void launch_histogram(const uint32_t* keys, const uint32_t* n_ptr, uint32_t n_cap, uint32_t* hist4x256,
                       cudaStream_t st);
-void launch_set_count(uint32_t* dst, uint32_t value, cudaStream_t st);
 void launch_lookback_probe(uint64_t* status, uint32_t* err, uint32_t spin_limit, uint32_t* out, cudaStream_t st);
 
 }  // namespace spl
