@@ -29,6 +29,7 @@ namespace spl {
 constexpr int GR = 10;  // gradient words per record
 
 __global__ void k_zero_grad_rec(float* grad_rec, const FrameCounters* fc, uint32_t* deferred) {
+    frame_step();
     if (blockIdx.x == 0 && threadIdx.x == 0) deferred[0] = 0u;
     const uint32_t n = fc->visible * GR;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) grad_rec[i] = 0.0f;
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restr
     __shared__ uint8_t s_list[8][8][RASTER_BATCH];                   // [warp][group]
     const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5, lt = lanemask_lt();
     const uint32_t grp = lane >> 2, li = lane & 3u;
+    frame_step(ranges, tile_order, pair_vals, rec, image, grad_image);
     // the forward's most-pairs-first order of this frame's tiles, when it made one
     uint2 rg;
     int tile;
@@ -305,6 +307,7 @@ __global__ void __launch_bounds__(128, 4) k_preprocess_backward(SceneView s, Uni
                                                              float* gz, float4* grot, float4* gscale_alpha,
                                                              float* gsh, uint32_t* deferred, uint32_t deferred_cap,
                                                              bool accumulate) {
+    frame_step(idx, fc, boxes, grad_rec);
     const uint32_t V = fc->visible;
     for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < V; slot += gridDim.x * blockDim.x) {
         float g[GR];
@@ -357,6 +360,7 @@ __global__ void __launch_bounds__(128) k_preprocess_backward_double(SceneView s,
                                                                     float4* gscale_alpha,
                                                                     const uint32_t* __restrict__ deferred,
                                                                     uint32_t deferred_cap, bool accumulate) {
+    frame_step(idx, boxes, grad_rec, deferred);
     const uint32_t n = min(deferred[0], deferred_cap);
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const uint32_t slot = deferred[1 + k];
@@ -385,14 +389,14 @@ void launch_backward(int sh_order, bool covariance, bool rect, const SceneView& 
     uint32_t zg = (max_n * GR + 255) / 256;
     if (zg > device_sm_count() * 8u) zg = device_sm_count() * 8u;
     if (zg == 0) zg = 1;
-    k_zero_grad_rec<<<zg, 256, 0, st>>>(grad_rec, fc, deferred);
+    launch_after(k_zero_grad_rec, zg, 256, st, grad_rec, fc, deferred);
     const int grid = tiles_x * tiles_y;
     if (!raster_orders_tiles((uint64_t)grid)) tile_order = nullptr;
     if (grid > 0) {
         auto k = !rect ? k_raster_backward<false, true>
                        : (fabsf(u.margin) <= RASTER_NEAR_MARGIN ? k_raster_backward<true, false> : k_raster_backward<true, true>);
-        k<<<grid, 256, 0, st>>>(ranges, tile_order, pair_vals, rec, W, H, tiles_x, u.margin, psx, psy, image, grad_image,
-                                grad_rec);
+        launch_after(k, (uint32_t)grid, 256, st, ranges, tile_order, pair_vals, rec, W, H, tiles_x, u.margin, psx, psy, image,
+                     grad_image, grad_rec);
     }
     if (max_n == 0) return;
     uint32_t blocks = (max_n + 127) / 128;
@@ -401,11 +405,10 @@ void launch_backward(int sh_order, bool covariance, bool rect, const SceneView& 
     const uint32_t dblocks = device_sm_count() * 2u;
 #define PB(SHO, COV)                                                                                          \
     do {                                                                                                      \
-        k_preprocess_backward<SHO, COV><<<blocks, 128, 0, st>>>(s, u, idx, fc, boxes, grad_rec, gx, gy, gz, grot, \
-                                                                gscale_alpha, gsh, deferred, max_n, accumulate); \
-        k_preprocess_backward_double<SHO, COV><<<dblocks, 128, 0, st>>>(s, u, idx, boxes, grad_rec, gx, gy, gz,   \
-                                                                        grot, gscale_alpha, deferred, max_n,      \
-                                                                        accumulate);                              \
+        launch_after(k_preprocess_backward<SHO, COV>, blocks, 128, st, s, u, idx, fc, boxes, grad_rec, gx, gy, gz, \
+                     grot, gscale_alpha, gsh, deferred, max_n, accumulate);                                        \
+        launch_after(k_preprocess_backward_double<SHO, COV>, dblocks, 128, st, s, u, idx, boxes, grad_rec, gx, gy, \
+                     gz, grot, gscale_alpha, deferred, max_n, accumulate);                                         \
     } while (0)
     switch (sh_order * 2 + (covariance ? 1 : 0)) {
         case 0: PB(0, false); break;
