@@ -263,6 +263,11 @@ struct VjpInputs {
         rx = Xr * ((2.0f * vw) / (float)u.image_size[0]) - vw;
         ry = vh - Yr * ((2.0f * vh) / (float)u.image_size[1]);
     }
+    template <class T, bool COV, int PARTS>
+    __device__ __forceinline__ void vjp(const Uniforms& u, const float* g, T* gin) const {
+        vertex_vjp_t<T, SHO, COV, PARTS>(u, cx, cy, cz, rot.x, rot.y, rot.z, rot.w, sca.x, sca.y, sca.z, sh, rx, ry, g,
+                                             gin);
+    }
 };
 
 __device__ __forceinline__ bool load_record_gradient(const float* grad_rec, uint32_t slot, float* g) {
@@ -320,8 +325,9 @@ __global__ void __launch_bounds__(128, 4) k_preprocess_backward(SceneView s, Uni
             if (pos < deferred_cap) deferred[1 + pos] = slot;
         } else {
             float gin[10];
-            vertex_vjp_t<float, SHO, COV>(u, in.cx, in.cy, in.cz, in.rot.x, in.rot.y, in.rot.z, in.rot.w, in.sca.x,
-                                          in.sca.y, in.sca.z, in.sh, in.rx, in.ry, g, gin);
+            in.template vjp<float, COV, VJP_ALL>(u, g, gin);
+#pragma unroll
+            for (int m = 0; m < 10; ++m) gin[m] = finite_gradient(gin[m]);
             store_splat_gradient(i, gin, g[6], gx, gy, gz, grot, gscale_alpha, accumulate);
         }
         // SH: rgb_c = 0.5 + sum_k B_k(d) sh[3k + c]
@@ -350,9 +356,15 @@ __global__ void __launch_bounds__(128, 4) k_preprocess_backward(SceneView s, Uni
     }
 }
 
-// The deferred needles and discs, swept in double (same formulas, same float forward values).
+// The deferred needles and discs, swept in double (same formulas, same float forward values).  
+// A double operation holds its scheduler's pipe for some 30 cycles whatever the number of lanes, so that even one
+// splat's sweep, some 2000 of them one after another, took 65 us, as long as the float sweep of 500k splats; fused
+// products and shared reciprocals take it to 41 us.  A block takes 32 splats, a warp each for the gradients' three
+// parts: 26 us.  (Computing what the parts share again costs more than it gives above some 40k needles: 150k of 1M
+// splats, eight views' backward 3338 us, 2980 us with a thread per splat, 3420 us before; a branch to that in the same
+// kernel makes the few needles' sweep 36 us.)
 template <int SHO, bool COV>
-__global__ void __launch_bounds__(128) k_preprocess_backward_double(SceneView s, Uniforms u,
+__global__ void __launch_bounds__(96) k_preprocess_backward_double(SceneView s, Uniforms u,
                                                                     const uint32_t* __restrict__ idx,
                                                                     const uint2* __restrict__ boxes,
                                                                     const float* __restrict__ grad_rec, float* gx,
@@ -362,17 +374,38 @@ __global__ void __launch_bounds__(128) k_preprocess_backward_double(SceneView s,
                                                                     uint32_t deferred_cap, bool accumulate) {
     frame_step(idx, boxes, grad_rec, deferred);
     const uint32_t n = min(deferred[0], deferred_cap);
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const uint32_t slot = deferred[1 + k];
+    __shared__ double s_part[2][10][32];
+    const uint32_t lane = threadIdx.x & 31u, part = threadIdx.x >> 5;
+    for (uint32_t k0 = blockIdx.x * 32u; k0 < n; k0 += gridDim.x * 32u) {
+        const uint32_t k = k0 + lane;
         float g[GR];
-        load_record_gradient(grad_rec, slot, g);
-        const uint32_t i = __ldg(idx + slot);
-        VjpInputs<SHO> in;
-        in.load(s, u, i, __ldg(boxes + slot));
-        float gin[10];
-        vertex_vjp_t<double, SHO, COV>(u, in.cx, in.cy, in.cz, in.rot.x, in.rot.y, in.rot.z, in.rot.w, in.sca.x,
-                                       in.sca.y, in.sca.z, in.sh, in.rx, in.ry, g, gin);
-        store_splat_gradient(i, gin, g[6], gx, gy, gz, grot, gscale_alpha, accumulate);
+        double gin[10];
+        uint32_t i = 0;
+        if (k < n) {
+            const uint32_t slot = deferred[1 + k];
+            load_record_gradient(grad_rec, slot, g);
+            i = __ldg(idx + slot);
+            VjpInputs<SHO> in;
+            in.load(s, u, i, __ldg(boxes + slot));
+            if (part == 0)
+                in.template vjp<double, COV, VJP_OUTLINE>(u, g, gin);
+            else if (part == 1)
+                in.template vjp<double, COV, VJP_AXES>(u, g, gin);
+            else
+                in.template vjp<double, COV, VJP_COLOUR>(u, g, gin);
+            if (part != 0) {
+#pragma unroll
+                for (int m = 0; m < 10; ++m) s_part[part - 1][m][lane] = gin[m];
+            }
+        }
+        __syncthreads();
+        if (part == 0 && k < n) {
+            float sum[10];
+#pragma unroll
+            for (int m = 0; m < 10; ++m) sum[m] = finite_gradient(gin[m] + s_part[0][m][lane] + s_part[1][m][lane]);
+            store_splat_gradient(i, sum, g[6], gx, gy, gz, grot, gscale_alpha, accumulate);
+        }
+        __syncthreads();
     }
 }
 
@@ -407,7 +440,7 @@ void launch_backward(int sh_order, bool covariance, bool rect, const SceneView& 
     do {                                                                                                      \
         launch_after(k_preprocess_backward<SHO, COV>, blocks, 128, st, s, u, idx, fc, boxes, grad_rec, gx, gy, gz, \
                      grot, gscale_alpha, gsh, deferred, max_n, accumulate);                                        \
-        launch_after(k_preprocess_backward_double<SHO, COV>, dblocks, 128, st, s, u, idx, boxes, grad_rec, gx, gy, \
+        launch_after(k_preprocess_backward_double<SHO, COV>, dblocks, 96, st, s, u, idx, boxes, grad_rec, gx, gy, \
                      gz, grot, gscale_alpha, deferred, max_n, accumulate);                                         \
     } while (0)
     switch (sh_order * 2 + (covariance ? 1 : 0)) {

@@ -25,6 +25,30 @@ __device__ __forceinline__ float sign_(S x) {
 }
 
 // ---- mat3 (column-major m[c*3 + r]); (A*B) column j = A * B[j] in column order ------------------
+// Sums of products: in float each operation rounded (the oracle's arithmetic), in double fused, since a double
+// operation holds its pipe for tens of cycles a warp.
+template <class S>
+__device__ __forceinline__ S mad(S a, S b, S c) {
+    return a * b + c;
+}
+template <>
+__device__ __forceinline__ double mad(double a, double b, double c) {
+    return fma(a, b, c);
+}
+template <class S>
+__device__ __forceinline__ S dot2(S a, S b, S c, S d) {
+    return mad(a, b, c * d);
+}
+template <class S>
+__device__ __forceinline__ S dot3(S a, S b, S c, S d, S e, S f) {
+    return mad(e, f, mad(a, b, c * d));
+}
+// a / b; in double by the reciprocal ib, which is computed once for all quotients by b.
+__device__ __forceinline__ float over(float a, float b, float) { return a / b; }
+__device__ __forceinline__ double over(double a, double, double ib) { return a * ib; }
+__device__ __forceinline__ float reciprocal(float) { return 0.0f; }  // not used
+__device__ __forceinline__ double reciprocal(double b) { return 1.0 / b; }
+
 template <class S>
 struct M3T {
     S m[9];
@@ -36,7 +60,8 @@ __device__ __forceinline__ M3T<S> mul3(const M3T<S>& A, const M3T<S>& B) {
     for (int j = 0; j < 3; ++j)
 #pragma unroll
         for (int i = 0; i < 3; ++i)
-            t.m[j * 3 + i] = (A.m[0 * 3 + i] * B.m[j * 3 + 0] + A.m[1 * 3 + i] * B.m[j * 3 + 1]) + A.m[2 * 3 + i] * B.m[j * 3 + 2];
+            t.m[j * 3 + i] =
+                dot3(A.m[0 * 3 + i], B.m[j * 3 + 0], A.m[1 * 3 + i], B.m[j * 3 + 1], A.m[2 * 3 + i], B.m[j * 3 + 2]);
     return t;
 }
 template <class S>
@@ -328,25 +353,33 @@ __device__ __forceinline__ void sh_channel_grad(const float* sh, int c, T gc, T 
     if (SHO > 1) {
         const float k4 = c_shc[4] * sh[12 + c], k5 = c_shc[5] * sh[15 + c], k6 = c_shc[6] * sh[18 + c];
         const float k7 = c_shc[7] * sh[21 + c], k8 = c_shc[8] * sh[24 + c];
-        gx += (k4 * y + k7 * z) + (k8 - k6) * (2.0f * x);
-        gy += (k4 * x + k5 * z) - (k6 + k8) * (2.0f * y);
-        gz += (k5 * y + k7 * x) + k6 * (4.0f * z);
+        gx += dot3<T>(k4, y, k7, z, k8 - k6, 2.0f * x);
+        gy += dot3<T>(k4, x, k5, z, -(k6 + k8), 2.0f * y);
+        gz += dot3<T>(k5, y, k7, x, k6, 4.0f * z);
     }
     if (SHO > 2) {
         const float k9 = c_shc[9] * sh[27 + c], k10 = c_shc[10] * sh[30 + c], k11 = c_shc[11] * sh[33 + c];
         const float k12 = c_shc[12] * sh[36 + c], k13 = c_shc[13] * sh[39 + c], k14 = c_shc[14] * sh[42 + c];
         const float k15 = c_shc[15] * sh[45 + c];
         const float f11 = (4.0f * zz - xx) - yy;  // the factor of y (k11) and of x (k13)
-        gx += k9 * (6.0f * x * y) + k10 * (y * z) - k11 * (2.0f * x * y) - k12 * (6.0f * x * z) +
-              k13 * (f11 - 2.0f * xx) + k14 * (2.0f * x * z) + k15 * (3.0f * xx - 3.0f * yy);
-        gy += k9 * (3.0f * xx - 3.0f * yy) + k10 * (x * z) + k11 * (f11 - 2.0f * yy) - k12 * (6.0f * y * z) -
-              k13 * (2.0f * x * y) - k14 * (2.0f * y * z) - k15 * (6.0f * x * y);
-        gz += k10 * (x * y) + k11 * (8.0f * y * z) + k12 * ((2.0f * zz - 3.0f * xx) - 3.0f * yy + 4.0f * zz) +
-              k13 * (8.0f * x * z) + k14 * (xx - yy);
+        gx += mad<T>(k15, 3.0f * xx - 3.0f * yy,
+                     mad<T>(k14, 2.0f * x * z,
+                            mad<T>(k13, f11 - 2.0f * xx,
+                                   mad<T>(-k12, 6.0f * x * z,
+                                          mad<T>(-k11, 2.0f * x * y, dot2<T>(k9, 6.0f * x * y, k10, y * z))))));
+        gy += mad<T>(-k15, 6.0f * x * y,
+                     mad<T>(-k14, 2.0f * y * z,
+                            mad<T>(-k13, 2.0f * x * y,
+                                   mad<T>(-k12, 6.0f * y * z,
+                                          mad<T>(k11, f11 - 2.0f * yy, dot2<T>(k9, 3.0f * xx - 3.0f * yy, k10, x * z))))));
+        gz += mad<T>(k14, xx - yy,
+                     mad<T>(k13, 8.0f * x * z,
+                            mad<T>(k12, (2.0f * zz - 3.0f * xx) - 3.0f * yy + 4.0f * zz,
+                                   dot2<T>(k10, x * y, k11, 8.0f * y * z))));
     }
-    gd[0] += gc * gx;
-    gd[1] += gc * gy;
-    gd[2] += gc * gz;
+    gd[0] = mad(gc, gx, gd[0]);
+    gd[1] = mad(gc, gy, gd[1]);
+    gd[2] = mad(gc, gz, gd[2]);
 }
 
 // The vertex stage's vector-Jacobian product, in reverse mode: the gradients of the record's affine map
@@ -372,10 +405,14 @@ __device__ __forceinline__ void sh_channel_grad(const float* sh, int c, T gc, T 
 //   dpsi = V^T dE U / (U^T E U - V^T E V) (eigenvector perturbation);
 // * the covariance semi-axes (projected_covariance) through the eigenvectors of the projected 2x2;
 // * the rectangle basis and its inverse, and the SH colour of the view direction.
-template <class T, int SHO, bool COV>
+//
+// Every gradient is the sum of three parts, of the covariance semi-axes, of the outline and of the colour, which
+// share only values that are cheap to compute again: vertex_vjp_t gives the sum of the parts in PARTS.
+constexpr int VJP_AXES = 1, VJP_OUTLINE = 2, VJP_COLOUR = 4, VJP_ALL = 7;
+template <class T, int SHO, bool COV, int PARTS>
 __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float cyf, float czf, float q0f, float q1f,
                                              float q2f, float q3f, float scx, float scy, float scz, const float* sh,
-                                             float rxf, float ryf, const float* gf, float* gin) {
+                                             float rxf, float ryf, const float* gf, T* gin) {
     // the outline's centre and axes: the forward's float values
     float t0f, t1f, rjf, rkf, ax0f, ax1f;
     outline_ellipse<COV>(u, scx * u.splat_scale, scy * u.splat_scale, scz * u.splat_scale, q0f, q1f, q2f, q3f, cxf,
@@ -391,20 +428,20 @@ __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float
     const M3T<T> R = quat_to_mat(q0, q1, q2, q3);
     M3T<T> Ri;  // R^-1 by the adjugate over the determinant
     {
-        const T c00 = R.m[4] * R.m[8] - R.m[7] * R.m[5];
-        const T c01 = R.m[7] * R.m[2] - R.m[1] * R.m[8];
-        const T c02 = R.m[1] * R.m[5] - R.m[4] * R.m[2];
-        const T det = (R.m[0] * c00 + R.m[3] * c01) + R.m[6] * c02;
+        const T c00 = dot2(R.m[4], R.m[8], -R.m[7], R.m[5]);
+        const T c01 = dot2(R.m[7], R.m[2], -R.m[1], R.m[8]);
+        const T c02 = dot2(R.m[1], R.m[5], -R.m[4], R.m[2]);
+        const T det = dot3(R.m[0], c00, R.m[3], c01, R.m[6], c02);
         const T idet = 1.0f / det;
         Ri.m[0] = c00 * idet;
-        Ri.m[3] = (R.m[6] * R.m[5] - R.m[3] * R.m[8]) * idet;
-        Ri.m[6] = (R.m[3] * R.m[7] - R.m[6] * R.m[4]) * idet;
+        Ri.m[3] = dot2(R.m[6], R.m[5], -R.m[3], R.m[8]) * idet;
+        Ri.m[6] = dot2(R.m[3], R.m[7], -R.m[6], R.m[4]) * idet;
         Ri.m[1] = c01 * idet;
-        Ri.m[4] = (R.m[0] * R.m[8] - R.m[6] * R.m[2]) * idet;
-        Ri.m[7] = (R.m[6] * R.m[1] - R.m[0] * R.m[7]) * idet;
+        Ri.m[4] = dot2(R.m[0], R.m[8], -R.m[6], R.m[2]) * idet;
+        Ri.m[7] = dot2(R.m[6], R.m[1], -R.m[0], R.m[7]) * idet;
         Ri.m[2] = c02 * idet;
-        Ri.m[5] = (R.m[3] * R.m[2] - R.m[0] * R.m[5]) * idet;
-        Ri.m[8] = (R.m[0] * R.m[4] - R.m[3] * R.m[1]) * idet;
+        Ri.m[5] = dot2(R.m[3], R.m[2], -R.m[0], R.m[5]) * idet;
+        Ri.m[8] = dot2(R.m[0], R.m[4], -R.m[3], R.m[1]) * idet;
     }
     const M3T<T> K = mul3(Ri, C);
     const T s2[3] = {sx * sx, sy * sy, sz * sz};
@@ -412,16 +449,18 @@ __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float
     T Sg[6];  // Sigma: xx, xy, yy, xz, yz, zz (the first three only through N below)
 #pragma unroll
     for (int e = 3; e < 6; ++e)
-        Sg[e] = (s2[0] * m3(K, 0, ii[e])) * m3(K, 0, jj[e]) + (s2[1] * m3(K, 1, ii[e])) * m3(K, 1, jj[e]) +
-                (s2[2] * m3(K, 2, ii[e])) * m3(K, 2, jj[e]);
+        Sg[e] = dot3(s2[0] * m3(K, 0, ii[e]), m3(K, 0, jj[e]), s2[1] * m3(K, 1, ii[e]), m3(K, 1, jj[e]),
+                     s2[2] * m3(K, 2, ii[e]), m3(K, 2, jj[e]));
     const T ro[3] = {u.camera[12] - cx, u.camera[13] - cy, u.camera[14] - cz};
     T w[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) w[i] = (u.camera[i * 4 + 0] * ro[0] + u.camera[i * 4 + 1] * ro[1]) + u.camera[i * 4 + 2] * ro[2];
+    for (int i = 0; i < 3; ++i) 
+        w[i] = dot3<T>(u.camera[i * 4 + 0], ro[0], u.camera[i * 4 + 1], ro[1], u.camera[i * 4 + 2], ro[2]);
     const T Sxz = Sg[3], Syz = Sg[4], Szz = Sg[5];
     const T wz2 = w[2] * w[2];
     const T k = wz2 - Szz;
-    const T mx = (w[0] * w[2] - Sxz) / k, my = (w[1] * w[2] - Syz) / k;
+    const T ik = reciprocal(k);
+    const T mx = over(mad(w[0], w[2], -Sxz), k, ik), my = over(mad(w[1], w[2], -Syz), k, ik);
     // N = F - M without cancellation between the splat's scales:
     //   F = sum_a s_a^2 v_a v_a^T,  v_a = w_z K(a, xy) - K(a, z) w_xy   (Sigma_2 w_z^2 - w_z (w_2 s^T + s w_2^T) + Szz w_2 w_2^T)
     //   M = sum_{a<b} s_a^2 s_b^2 u_ab u_ab^T,  u_ab = K(b, z) K(a, xy) - K(a, z) K(b, xy)   (Sigma_2 Szz - s s^T, by
@@ -432,32 +471,32 @@ __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float
     T Nxx = 0.0f, Nxy = 0.0f, Nyy = 0.0f;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        va[a][0] = w[2] * m3(K, a, 0) - m3(K, a, 2) * w[0];
-        va[a][1] = w[2] * m3(K, a, 1) - m3(K, a, 2) * w[1];
-        Nxx += s2[a] * (va[a][0] * va[a][0]);
-        Nxy += s2[a] * (va[a][0] * va[a][1]);
-        Nyy += s2[a] * (va[a][1] * va[a][1]);
+        va[a][0] = dot2(w[2], m3(K, a, 0), -m3(K, a, 2), w[0]);
+        va[a][1] = dot2(w[2], m3(K, a, 1), -m3(K, a, 2), w[1]);
+        Nxx = mad(s2[a], va[a][0] * va[a][0], Nxx);
+        Nxy = mad(s2[a], va[a][0] * va[a][1], Nxy);
+        Nyy = mad(s2[a], va[a][1] * va[a][1], Nyy);
     }
 #pragma unroll
     for (int pq = 0; pq < 3; ++pq) {
         const int a = pa[pq], b = pb[pq];
-        uab[pq][0] = m3(K, b, 2) * m3(K, a, 0) - m3(K, a, 2) * m3(K, b, 0);
-        uab[pq][1] = m3(K, b, 2) * m3(K, a, 1) - m3(K, a, 2) * m3(K, b, 1);
+        uab[pq][0] = dot2(m3(K, b, 2), m3(K, a, 0), -m3(K, a, 2), m3(K, b, 0));
+        uab[pq][1] = dot2(m3(K, b, 2), m3(K, a, 1), -m3(K, a, 2), m3(K, b, 1));
         const T p = s2[a] * s2[b];
-        Nxx -= p * (uab[pq][0] * uab[pq][0]);
-        Nxy -= p * (uab[pq][0] * uab[pq][1]);
-        Nyy -= p * (uab[pq][1] * uab[pq][1]);
+        Nxx = mad(-p, uab[pq][0] * uab[pq][0], Nxx);
+        Nxy = mad(-p, uab[pq][0] * uab[pq][1], Nxy);
+        Nyy = mad(-p, uab[pq][1] * uab[pq][1], Nyy);
     }
-    const T ik2 = 1.0f / (k * k);
+    const T ik2 = over((T)1.0f, k * k, ik * ik);
     const T Exx = Nxx * ik2, Exy = Nxy * ik2, Eyy = Nyy * ik2;
     const T U0 = rk, U1 = -rj, V0 = rj, V1 = rk;
-    const T quu = ((U0 * U0) * Exx + (2.0f * (U0 * U1)) * Exy) + (U1 * U1) * Eyy;
-    const T qvv = ((V0 * V0) * Exx + (2.0f * (V0 * V1)) * Exy) + (V1 * V1) * Eyy;
+    const T quu = dot3(U0 * U0, Exx, 2.0f * (U0 * U1), Exy, U1 * U1, Eyy);
+    const T qvv = dot3(V0 * V0, Exx, 2.0f * (V0 * V1), Exy, V1 * V1, Eyy);
     const T gap = quu - qvv;
     const T r0 = sqrt(quu), r1 = sqrt(qvv);
     // covariance semi-axes (projected_covariance), values kept for the sweep back
     M3T<T> Q, Tm;
-    T v[3], v2 = 0.0f, zzv = 0.0f, qr[2] = {0.0f, 0.0f}, pxx = 0.0f, pxy = 0.0f, pyy = 0.0f, bsq = 0.0f;
+    T v[3], v2 = 0.0f, iv2 = 0.0f, zzv = 0.0f, qr[2] = {0.0f, 0.0f}, pxx = 0.0f, pxy = 0.0f, pyy = 0.0f, bsq = 0.0f;
     bool pass[2] = {false, false};
     if (COV) {
         M3T<T> Ts = R;  // R with its columns scaled
@@ -469,11 +508,12 @@ __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float
         }
 #pragma unroll
         for (int r = 0; r < 3; ++r)
-            v[r] = ((u.view[0 * 4 + r] * cx + u.view[1 * 4 + r] * cy) + u.view[2 * 4 + r] * cz) + u.view[3 * 4 + r] * 1.0f;
+            v[r] = dot3<T>(u.view[0 * 4 + r], cx, u.view[1 * 4 + r], cy, u.view[2 * 4 + r], cz) + u.view[3 * 4 + r] * 1.0f;
         v2 = v[2];
+        iv2 = reciprocal(v2);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const T q = v[i] / v2;
+            const T q = over(v[i], v2, iv2);
             const T mlo = fmax(q, (T)-1.0f), mhi = fmin(mlo, (T)1.0f);
             pass[i] = mlo == q && mhi == mlo;  // inside the clamp: the derivative follows q
             qr[i] = mhi;
@@ -481,8 +521,8 @@ __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float
         }
         zzv = v2 * v2;
         M3T<T> J;
-        J.m[0] = 1.0f / v2; J.m[1] = 0.0f; J.m[2] = (-v[0]) / zzv;
-        J.m[3] = 0.0f; J.m[4] = 1.0f / v2; J.m[5] = (-v[1]) / zzv;
+        J.m[0] = over((T)1.0f, v2, iv2); J.m[1] = 0.0f; J.m[2] = over(-v[0], zzv, iv2 * iv2);
+        J.m[3] = 0.0f; J.m[4] = over((T)1.0f, v2, iv2); J.m[5] = over(-v[1], zzv, iv2 * iv2);
         J.m[6] = 0.0f; J.m[7] = 0.0f; J.m[8] = 0.0f;
         Q = mul3(transpose3(Ts), C);
         Tm = mul3(Q, J);
@@ -491,14 +531,14 @@ __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float
         pxy = P.m[1];
         pyy = P.m[4];
         const T a = (pxx - pyy) * (pxx - pyy);
-        bsq = sqrt(a + (4.0f * pxy) * pxy);
+        bsq = sqrt(mad(4.0f * pxy, pxy, a));
         ax0 = sqrt(((pxx + pyy) + bsq) * 0.5f);
         ax1 = sqrt(((pxx + pyy) - bsq) * 0.5f);
     }
     // rectangle basis and its inverse
     const T sa = u.bias + ax0, sb = u.bias + ax1;
     const T Xx = rk * sa, Xy = (-rj) * sa, Yx = rj * sb, Yy = rk * sb;
-    const T det2 = Xx * Yy - Xy * Yx;
+    const T det2 = dot2(Xx, Yy, -Xy, Yx);
     const T idet2 = 1.0f / det2;
     const T i00 = Yy * idet2, i01 = (-Yx) * idet2, i10 = (-Xy) * idet2, i11 = Xx * idet2;
     const T psx = (2.0f * u.view_size[0]) / (T)u.image_size[0];
@@ -506,36 +546,37 @@ __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float
     const T ox = rx - t0, oy = ry - t1;
 
     // ---- sweep back: affine map -> ellipse ----
-    const T bi00 = g[0] * psx + g[2] * ox, bi01 = g[1] * psy + g[2] * oy;
-    const T bi10 = g[3] * psx + g[5] * ox, bi11 = g[4] * psy + g[5] * oy;
-    const T bt0 = -(g[2] * i00 + g[5] * i10), bt1 = -(g[2] * i01 + g[5] * i11);
+    const T bi00 = dot2(g[0], psx, g[2], ox), bi01 = dot2(g[1], psy, g[2], oy);
+    const T bi10 = dot2(g[3], psx, g[5], ox), bi11 = dot2(g[4], psy, g[5], oy);
+    const T bt0 = -dot2(g[2], i00, g[5], i10), bt1 = -dot2(g[2], i01, g[5], i11);
     T bXx = bi11 * idet2, bXy = -(bi10 * idet2), bYx = -(bi01 * idet2), bYy = bi00 * idet2;
-    const T bidet = ((bi00 * Yy - bi01 * Yx) - bi10 * Xy) + bi11 * Xx;
+    const T bidet = mad(bi11, Xx, mad(-bi10, Xy, dot2(bi00, Yy, -bi01, Yx)));
     const T bdet = bidet * (-(idet2 * idet2));
-    bXx += bdet * Yy;
-    bYy += bdet * Xx;
-    bXy -= bdet * Yx;
-    bYx -= bdet * Xy;
-    const T brk = bXx * sa + bYy * sb, brj = bYx * sb - bXy * sa;
-    const T bax0 = bXx * rk - bXy * rj, bax1 = bYx * rj + bYy * rk;
+    bXx = mad(bdet, Yy, bXx);
+    bYy = mad(bdet, Xx, bYy);
+    bXy = mad(-bdet, Yx, bXy);
+    bYx = mad(-bdet, Xy, bYx);
+    const T brk = dot2(bXx, sa, bYy, sb), brj = dot2(bYx, sb, -bXy, sa);
+    const T bax0 = dot2(bXx, rk, -bXy, rj), bax1 = dot2(bYx, rj, bYy, rk);
 
     T gc[3] = {0.0f, 0.0f, 0.0f}, gs[3] = {0.0f, 0.0f, 0.0f};
     M3T<T> bR;
 #pragma unroll
     for (int e = 0; e < 9; ++e) bR.m[e] = 0.0f;
     // ---- covariance semi-axes ----
-    if (COV) {
+    if (COV && (PARTS & VJP_AXES)) {
         // ax0^2, ax1^2 are the eigenvalues of the 2x2 (pxx pxy; pxy pyy); each eigenvalue's gradient is its
         // unit eigenvector's outer product (u for the larger, v for the smaller), which has none of the
         // cancellation of differentiating ((pxx + pyy) -+ b) / 2 for a needle's thin axis
         const T bh0 = ax0 > 0.0f ? bax0 / (2.0f * ax0) : 0.0f, bh1 = ax1 > 0.0f ? bax1 / (2.0f * ax1) : 0.0f;
         T bpxx, bpyy, bpxy;
         if (bsq > 0.0f) {
-            const T c2 = (pxx - pyy) / bsq, sn2 = (2.0f * pxy) / bsq;  // cos, sin of twice the axis angle
+            const T ib = reciprocal(bsq);
+            const T c2 = over(pxx - pyy, bsq, ib), sn2 = over(2.0f * pxy, bsq, ib);  // cos, sin of twice the axis angle
             const T cu = sqrt(fmax((T)0.0f, (T)0.5f * ((T)1.0f + c2)));
             const T su = copysign(sqrt(fmax((T)0.0f, (T)0.5f * ((T)1.0f - c2))), sn2);
-            bpxx = bh0 * (cu * cu) + bh1 * (su * su);
-            bpyy = bh0 * (su * su) + bh1 * (cu * cu);
+            bpxx = dot2(bh0, cu * cu, bh1, su * su);
+            bpyy = dot2(bh0, su * su, bh1, cu * cu);
             bpxy = 2.0f * (bh0 - bh1) * (cu * su);
         } else {  // equal eigenvalues: the derivative the formula takes there (b's derivative is zero)
             bpxx = bpyy = 0.5f * (bh0 + bh1);
@@ -545,75 +586,77 @@ __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float
         M3T<T> bTm;
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
-            bTm.m[0 * 3 + r] = 2.0f * bpxx * m3(Tm, r, 0) + bpxy * m3(Tm, r, 1);
-            bTm.m[1 * 3 + r] = 2.0f * bpyy * m3(Tm, r, 1) + bpxy * m3(Tm, r, 0);
+            bTm.m[0 * 3 + r] = dot2(2.0f * bpxx, m3(Tm, r, 0), bpxy, m3(Tm, r, 1));
+            bTm.m[1 * 3 + r] = dot2(2.0f * bpyy, m3(Tm, r, 1), bpxy, m3(Tm, r, 0));
             bTm.m[2 * 3 + r] = 0.0f;
         }
         // Tm = Q J: bQ = bTm J^T, bJ = Q^T bTm (only J's non-zero entries matter)
-        const T J00 = 1.0f / v2, J20 = (-v[0]) / zzv, J21 = (-v[1]) / zzv;
+        const T iv4 = iv2 * iv2;
+        const T J00 = over((T)1.0f, v2, iv2), J20 = over(-v[0], zzv, iv4), J21 = over(-v[1], zzv, iv4);
         M3T<T> bQ;
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
             bQ.m[0 * 3 + r] = m3(bTm, r, 0) * J00;           // J(0, 0)
             bQ.m[1 * 3 + r] = m3(bTm, r, 1) * J00;           // J(1, 1)
-            bQ.m[2 * 3 + r] = m3(bTm, r, 0) * J20 + m3(bTm, r, 1) * J21;
+            bQ.m[2 * 3 + r] = dot2(m3(bTm, r, 0), J20, m3(bTm, r, 1), J21);
         }
         T bJ00 = 0.0f, bJ11 = 0.0f, bJ20 = 0.0f, bJ21 = 0.0f;
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
-            bJ00 += m3(Q, r, 0) * m3(bTm, r, 0);
-            bJ11 += m3(Q, r, 1) * m3(bTm, r, 1);
-            bJ20 += m3(Q, r, 2) * m3(bTm, r, 0);
-            bJ21 += m3(Q, r, 2) * m3(bTm, r, 1);
+            bJ00 = mad(m3(Q, r, 0), m3(bTm, r, 0), bJ00);
+            bJ11 = mad(m3(Q, r, 1), m3(bTm, r, 1), bJ11);
+            bJ20 = mad(m3(Q, r, 2), m3(bTm, r, 0), bJ20);
+            bJ21 = mad(m3(Q, r, 2), m3(bTm, r, 1), bJ21);
         }
         T bv[3] = {0.0f, 0.0f, 0.0f};
-        bv[2] -= (bJ00 + bJ11) / (v2 * v2);
-        const T bzz = (bJ20 * v[0] + bJ21 * v[1]) / (zzv * zzv);
-        bv[2] += bzz * (2.0f * v2);
-        const T bvc[2] = {-(bJ20 / zzv), -(bJ21 / zzv)};
+        bv[2] -= over(bJ00 + bJ11, v2 * v2, iv4);
+        const T bzz = over(dot2(bJ20, v[0], bJ21, v[1]), zzv * zzv, iv4 * iv4);
+        bv[2] = mad(bzz, 2.0f * v2, bv[2]);
+        const T bvc[2] = {-over(bJ20, zzv, iv4), -over(bJ21, zzv, iv4)};
 #pragma unroll
         for (int i = 0; i < 2; ++i) {  // v_i = clamp(v_i / v2, -1, 1) v2
             const T bm = bvc[i] * v2;
-            bv[2] += bvc[i] * qr[i];
+            bv[2] = mad(bvc[i], qr[i], bv[2]);
             if (pass[i]) {
-                bv[i] += bm / v2;
-                bv[2] -= bm * qr[i] / v2;
+                bv[i] += over(bm, v2, iv2);
+                bv[2] -= over(bm * qr[i], v2, iv2);
             }
         }
 #pragma unroll
-        for (int i = 0; i < 3; ++i) gc[i] += (u.view[i * 4 + 0] * bv[0] + u.view[i * 4 + 1] * bv[1]) + u.view[i * 4 + 2] * bv[2];
+        for (int i = 0; i < 3; ++i)
+            gc[i] += dot3<T>(u.view[i * 4 + 0], bv[0], u.view[i * 4 + 1], bv[1], u.view[i * 4 + 2], bv[2]);
         // Q = T^T C: bT(m, i) = sum_j bQ(i, j) C(m, j); T(:, a) = R(:, a) s_a
         const T sc[3] = {sx, sy, sz};
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int mm = 0; mm < 3; ++mm) {
-                const T bT = (m3(bQ, a, 0) * m3(C, mm, 0) + m3(bQ, a, 1) * m3(C, mm, 1)) + m3(bQ, a, 2) * m3(C, mm, 2);
-                bR.m[a * 3 + mm] += bT * sc[a];
-                gs[a] += bT * m3(R, mm, a);
+                const T bT = dot3(m3(bQ, a, 0), m3(C, mm, 0), m3(bQ, a, 1), m3(C, mm, 1), m3(bQ, a, 2), m3(C, mm, 2));
+                bR.m[a * 3 + mm] = mad(bT, sc[a], bR.m[a * 3 + mm]);
+                gs[a] = mad(bT, m3(R, mm, a), gs[a]);
             }
     }
     // ---- the outline through the dual conic ----
-    {
+    if (PARTS & VJP_OUTLINE) {
         const T bmx = bt0, bmy = bt1;
-        const T bpsi = brk * rj - brj * rk;
+        const T bpsi = dot2(brk, rj, -brj, rk);
         const T bquv = gap != 0.0f ? bpsi / gap : 0.0f;
         const T bquu = (!COV && r0 > 0.0f) ? bax0 / (2.0f * r0) : 0.0f;
         const T bqvv = (!COV && r1 > 0.0f) ? bax1 / (2.0f * r1) : 0.0f;
-        const T bExx = (bquu * (U0 * U0) + bqvv * (V0 * V0)) + bquv * (U0 * V0);
-        const T bExy = (bquu * (2.0f * (U0 * U1)) + bqvv * (2.0f * (V0 * V1))) + bquv * (U0 * V1 + U1 * V0);
-        const T bEyy = (bquu * (U1 * U1) + bqvv * (V1 * V1)) + bquv * (U1 * V1);
+        const T bExx = dot3(bquu, U0 * U0, bqvv, V0 * V0, bquv, U0 * V0);
+        const T bExy = dot3(bquu, 2.0f * (U0 * U1), bqvv, 2.0f * (V0 * V1), bquv, dot2(U0, V1, U1, V0));
+        const T bEyy = dot3(bquu, U1 * U1, bqvv, V1 * V1, bquv, U1 * V1);
         const T bNxx = bExx * ik2, bNxy = bExy * ik2, bNyy = bEyy * ik2;
-        const T bik2 = (bExx * Nxx + bExy * Nxy) + bEyy * Nyy;
-        T bk = bik2 * (-2.0f * ik2 / k);
+        const T bik2 = dot3(bExx, Nxx, bExy, Nxy, bEyy, Nyy);
+        T bk = bik2 * over(-2.0f * ik2, k, ik);
         T bw[3] = {0.0f, 0.0f, 0.0f}, bS[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};  // xx xy yy xz yz zz
         // centre
-        bw[0] += bmx * w[2] / k;
-        bw[1] += bmy * w[2] / k;
-        bw[2] += (bmx * w[0] + bmy * w[1]) / k;
-        bS[3] -= bmx / k;
-        bS[4] -= bmy / k;
-        bk -= (bmx * mx + bmy * my) / k;
+        bw[0] += over(bmx * w[2], k, ik);
+        bw[1] += over(bmy * w[2], k, ik);
+        bw[2] += over(dot2(bmx, w[0], bmy, w[1]), k, ik);
+        bS[3] -= over(bmx, k, ik);
+        bS[4] -= over(bmy, k, ik);
+        bk -= over(dot2(bmx, mx, bmy, my), k, ik);
         // N = F - M (above): back to the scales, K and w
         M3T<T> bK;
 #pragma unroll
@@ -621,52 +664,51 @@ __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float
         T bs2[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            bs2[a] += (bNxx * (va[a][0] * va[a][0]) + bNxy * (va[a][0] * va[a][1])) + bNyy * (va[a][1] * va[a][1]);
-            const T bv0 = s2[a] * (2.0f * bNxx * va[a][0] + bNxy * va[a][1]);
-            const T bv1 = s2[a] * (2.0f * bNyy * va[a][1] + bNxy * va[a][0]);
-            bw[2] += bv0 * m3(K, a, 0) + bv1 * m3(K, a, 1);
-            bK.m[0 * 3 + a] += w[2] * bv0;
-            bK.m[1 * 3 + a] += w[2] * bv1;
-            bK.m[2 * 3 + a] -= bv0 * w[0] + bv1 * w[1];
-            bw[0] -= m3(K, a, 2) * bv0;
-            bw[1] -= m3(K, a, 2) * bv1;
+            bs2[a] += dot3(bNxx, va[a][0] * va[a][0], bNxy, va[a][0] * va[a][1], bNyy, va[a][1] * va[a][1]);
+            const T bv0 = s2[a] * dot2(2.0f * bNxx, va[a][0], bNxy, va[a][1]);
+            const T bv1 = s2[a] * dot2(2.0f * bNyy, va[a][1], bNxy, va[a][0]);
+            bw[2] += dot2(bv0, m3(K, a, 0), bv1, m3(K, a, 1));
+            bK.m[0 * 3 + a] = mad(w[2], bv0, bK.m[0 * 3 + a]);
+            bK.m[1 * 3 + a] = mad(w[2], bv1, bK.m[1 * 3 + a]);
+            bK.m[2 * 3 + a] -= dot2(bv0, w[0], bv1, w[1]);
+            bw[0] = mad(-m3(K, a, 2), bv0, bw[0]);
+            bw[1] = mad(-m3(K, a, 2), bv1, bw[1]);
         }
 #pragma unroll
         for (int pq = 0; pq < 3; ++pq) {
             const int a = pa[pq], b = pb[pq];
             const T p = s2[a] * s2[b];
-            const T bp = -((bNxx * (uab[pq][0] * uab[pq][0]) + bNxy * (uab[pq][0] * uab[pq][1])) +
-                               bNyy * (uab[pq][1] * uab[pq][1]));
-            bs2[a] += bp * s2[b];
-            bs2[b] += bp * s2[a];
-            const T bu0 = -p * (2.0f * bNxx * uab[pq][0] + bNxy * uab[pq][1]);
-            const T bu1 = -p * (2.0f * bNyy * uab[pq][1] + bNxy * uab[pq][0]);
-            bK.m[2 * 3 + b] += bu0 * m3(K, a, 0) + bu1 * m3(K, a, 1);
-            bK.m[0 * 3 + a] += m3(K, b, 2) * bu0;
-            bK.m[1 * 3 + a] += m3(K, b, 2) * bu1;
-            bK.m[2 * 3 + a] -= bu0 * m3(K, b, 0) + bu1 * m3(K, b, 1);
-            bK.m[0 * 3 + b] -= m3(K, a, 2) * bu0;
-            bK.m[1 * 3 + b] -= m3(K, a, 2) * bu1;
+            const T bp = -dot3(bNxx, uab[pq][0] * uab[pq][0], bNxy, uab[pq][0] * uab[pq][1], bNyy, uab[pq][1] * uab[pq][1]);
+            bs2[a] = mad(bp, s2[b], bs2[a]);
+            bs2[b] = mad(bp, s2[a], bs2[b]);
+            const T bu0 = -p * dot2(2.0f * bNxx, uab[pq][0], bNxy, uab[pq][1]);
+            const T bu1 = -p * dot2(2.0f * bNyy, uab[pq][1], bNxy, uab[pq][0]);
+            bK.m[2 * 3 + b] += dot2(bu0, m3(K, a, 0), bu1, m3(K, a, 1));
+            bK.m[0 * 3 + a] = mad(m3(K, b, 2), bu0, bK.m[0 * 3 + a]);
+            bK.m[1 * 3 + a] = mad(m3(K, b, 2), bu1, bK.m[1 * 3 + a]);
+            bK.m[2 * 3 + a] -= dot2(bu0, m3(K, b, 0), bu1, m3(K, b, 1));
+            bK.m[0 * 3 + b] = mad(-m3(K, a, 2), bu0, bK.m[0 * 3 + b]);
+            bK.m[1 * 3 + b] = mad(-m3(K, a, 2), bu1, bK.m[1 * 3 + b]);
         }
-        gs[0] += bs2[0] * (2.0f * sx);
-        gs[1] += bs2[1] * (2.0f * sy);
-        gs[2] += bs2[2] * (2.0f * sz);
+        gs[0] = mad(bs2[0], 2.0f * sx, gs[0]);
+        gs[1] = mad(bs2[1], 2.0f * sy, gs[1]);
+        gs[2] = mad(bs2[2], 2.0f * sz, gs[2]);
         // k = wz2 - Szz, wz2 = w2^2
         T bwz2 = bk;
         bS[5] -= bk;
-        bw[2] += bwz2 * (2.0f * w[2]);
+        bw[2] = mad(bwz2, 2.0f * w[2], bw[2]);
         // w_i = sum_r C(r, i) (camera_r - c_r)
 #pragma unroll
-        for (int r = 0; r < 3; ++r) gc[r] -= (bw[0] * m3(C, r, 0) + bw[1] * m3(C, r, 1)) + bw[2] * m3(C, r, 2);
+        for (int r = 0; r < 3; ++r) gc[r] -= dot3(bw[0], m3(C, r, 0), bw[1], m3(C, r, 1), bw[2], m3(C, r, 2));
         // Sigma_e = sum_a s2_a K(a, i_e) K(a, j_e) (only xz, yz and zz are left with adjoints)
 #pragma unroll
         for (int e = 3; e < 6; ++e)
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 const T kai = m3(K, a, ii[e]), kaj = m3(K, a, jj[e]);
-                gs[a] += bS[e] * (kai * kaj) * (2.0f * (a == 0 ? sx : (a == 1 ? sy : sz)));
-                bK.m[ii[e] * 3 + a] += bS[e] * s2[a] * kaj;
-                bK.m[jj[e] * 3 + a] += bS[e] * s2[a] * kai;
+                gs[a] = mad(bS[e] * (kai * kaj), 2.0f * (a == 0 ? sx : (a == 1 ? sy : sz)), gs[a]);
+                bK.m[ii[e] * 3 + a] = mad(bS[e] * s2[a], kaj, bK.m[ii[e] * 3 + a]);
+                bK.m[jj[e] * 3 + a] = mad(bS[e] * s2[a], kai, bK.m[jj[e] * 3 + a]);
             }
         // K = Ri C: bRi(r, kk) = sum_c bK(r, c) C(kk, c); Ri = R^-1: bR -= Ri^T bRi Ri^T
         M3T<T> bRi;
@@ -674,7 +716,8 @@ __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float
         for (int r = 0; r < 3; ++r)
 #pragma unroll
             for (int kk = 0; kk < 3; ++kk)
-                bRi.m[kk * 3 + r] = (m3(bK, r, 0) * m3(C, kk, 0) + m3(bK, r, 1) * m3(C, kk, 1)) + m3(bK, r, 2) * m3(C, kk, 2);
+                bRi.m[kk * 3 + r] = 
+                    dot3(m3(bK, r, 0), m3(C, kk, 0), m3(bK, r, 1), m3(C, kk, 1), m3(bK, r, 2), m3(C, kk, 2));
         const M3T<T> X1 = mul3(transpose3(Ri), bRi);
         const M3T<T> X2 = mul3(X1, transpose3(Ri));
 #pragma unroll
@@ -685,37 +728,41 @@ __device__ __forceinline__ void vertex_vjp_t(const Uniforms& u, float cxf, float
         const T s2c = (T)1.41421356237309504880f;  // quat_to_mat's float constant
         const T qx = q0 * s2c, qy = q1 * s2c, qz = q2 * s2c, qw = q3 * s2c;
         const T* b = bR.m;
-        const T gqx = ((b[1] - b[3]) * qw + (b[6] - b[2]) * qz) + (b[5] - b[7]) * qy;
-        const T gqy = ((b[1] + b[3]) * qz + (b[2] + b[6]) * qw) + (b[5] - b[7]) * qx - 2.0f * qy * (b[4] + b[8]);
-        const T gqz = ((b[1] + b[3]) * qy + (b[5] + b[7]) * qw) + (b[6] - b[2]) * qx - 2.0f * qz * (b[0] + b[8]);
-        const T gqw = ((b[1] - b[3]) * qx + (b[2] + b[6]) * qy) + (b[5] + b[7]) * qz - 2.0f * qw * (b[0] + b[4]);
-        gin[3] = (float)(gqx * s2c);
-        gin[4] = (float)(gqy * s2c);
-        gin[5] = (float)(gqz * s2c);
-        gin[6] = (float)(gqw * s2c);
+        const T gqx = dot3(b[1] - b[3], qw, b[6] - b[2], qz, b[5] - b[7], qy);
+        const T gqy = mad(-2.0f * qy, b[4] + b[8], dot3(b[1] + b[3], qz, b[2] + b[6], qw, b[5] - b[7], qx));
+        const T gqz = mad(-2.0f * qz, b[0] + b[8], dot3(b[1] + b[3], qy, b[5] + b[7], qw, b[6] - b[2], qx));
+        const T gqw = mad(-2.0f * qw, b[0] + b[4], dot3(b[1] - b[3], qx, b[2] + b[6], qy, b[5] + b[7], qz));
+        gin[3] = gqx * s2c;
+        gin[4] = gqy * s2c;
+        gin[5] = gqz * s2c;
+        gin[6] = gqw * s2c;
     }
     // ---- colour of the view direction ----
-    {
+    if (PARTS & VJP_COLOUR) {
         const T vx = cx - u.camera[12], vy = cy - u.camera[13], vz = cz - u.camera[14];
-        const T len = sqrt((vx * vx + vy * vy) + vz * vz);
-        const T dx = vx / len, dy = vy / len, dz = vz / len;
+        const T len = sqrt(dot3(vx, vx, vy, vy, vz, vz)), il = reciprocal(len);
+        const T dx = over(vx, len, il), dy = over(vy, len, il), dz = over(vz, len, il);
         T gd[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (int c = 0; c < 3; ++c)
             sh_channel_grad<SHO, T>(sh, c, g[7 + c], dx, dy, dz, dx * dx, dy * dy, dz * dz, gd);
-        const T dd = (dx * gd[0] + dy * gd[1]) + dz * gd[2];
-        gc[0] += (gd[0] - dx * dd) / len;
-        gc[1] += (gd[1] - dy * dd) / len;
-        gc[2] += (gd[2] - dz * dd) / len;
+        const T dd = dot3(dx, gd[0], dy, gd[1], dz, gd[2]);
+        gc[0] += over(mad(-dx, dd, gd[0]), len, il);
+        gc[1] += over(mad(-dy, dd, gd[1]), len, il);
+        gc[2] += over(mad(-dz, dd, gd[2]), len, il);
     }
-    gin[0] = (float)gc[0];
-    gin[1] = (float)gc[1];
-    gin[2] = (float)gc[2];
-    gin[7] = (float)(gs[0] * u.splat_scale);
-    gin[8] = (float)(gs[1] * u.splat_scale);
-    gin[9] = (float)(gs[2] * u.splat_scale);
-#pragma unroll
-    for (int i = 0; i < 10; ++i) gin[i] = isfinite(gin[i]) ? gin[i] : 0.0f;
+    gin[0] = gc[0];
+    gin[1] = gc[1];
+    gin[2] = gc[2];
+    gin[7] = gs[0] * u.splat_scale;
+    gin[8] = gs[1] * u.splat_scale;
+    gin[9] = gs[2] * u.splat_scale;
+}
+
+template <class T>
+__device__ __forceinline__ float finite_gradient(T g) {
+    const float f = (float)g;
+    return isfinite(f) ? f : 0.0f;
 }
 
 // Splats whose largest scale exceeds NEEDLE_RATIO times their smallest (needles and discs).  A rotation
