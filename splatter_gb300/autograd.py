@@ -32,10 +32,12 @@ def _ptr(t):
     return t.data_ptr()
 
 
-def _planes(t, n):
-    """The addresses of a contiguous (3, n) float32 tensor's rows."""
-    p = t.data_ptr()
-    return p, p + 4 * n, p + 8 * n
+def _planes(t):
+    """The addresses of t[0], t[1] and t[2], without the views; an IndexError where one of them is missing."""
+    p, row = t.data_ptr(), t.element_size() * t.stride(0)
+    if t.shape[0] < 3:
+        raise IndexError(f"three planes expected, got {t.shape[0]}")
+    return p, p + row, p + 2 * row
 
 
 class _Splats:
@@ -98,7 +100,7 @@ class _RenderSplats:  # built lazily so that importing the package does not impo
                     scale_alpha = scale_alpha.contiguous()
                     sh = sh.contiguous()
                     n = rot.shape[0]
-                    scene = _WrappedScene(renderer, n, _planes(xyz, n), _ptr(rot), _ptr(scale_alpha), _ptr(sh),
+                    scene = _WrappedScene(renderer, n, _planes(xyz), _ptr(rot), _ptr(scale_alpha), _ptr(sh),
                                           (xyz, rot, scale_alpha, sh))
                     img = renderer.render_frame(scene, camera_to_world, width, height)
                     ctx.renderer = renderer
@@ -121,7 +123,7 @@ class _RenderSplats:  # built lazily so that importing the package does not impo
                     gsh = torch.zeros_like(sh)
                     g = grad_img.contiguous().float()
                     check(r._lib.spl_render_backward(r.handle, ctx.scene.handle, _ptr(img), _ptr(g),
-                                                     *_planes(gxyz, rot.shape[0]), _ptr(grot), _ptr(gsa), _ptr(gsh),
+                                                     *_planes(gxyz), _ptr(grot), _ptr(gsa), _ptr(gsh),
                                                      _stream_ptr(None)))
                     return gxyz, grot, gsa, gsh, None, None, None, None
 
@@ -276,7 +278,7 @@ def activate_native(means, quats, log_scales, opacity_logits):
     f32 = dict(device=quats.device, dtype=torch.float32)
     xyz, rot, sa = torch.empty((3, n), **f32), torch.empty((n, 4), **f32), torch.empty((n, 4), **f32)
     check(_lib.load().spl_activate_splats(n, _ptr(means), _ptr(quats), _ptr(log_scales), _ptr(opacity_logits),
-                                          *_planes(xyz, n), _ptr(rot), _ptr(sa),
+                                          *_planes(xyz), _ptr(rot), _ptr(sa),
                                           _stream_ptr(None)))
     return xyz, rot, sa
 
