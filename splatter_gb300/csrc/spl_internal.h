@@ -37,6 +37,7 @@ inline int fail(int code, const char* fmt, ...) {
 constexpr uint64_t MAX_COUNT = (1ull << 30) - 1;  // look-back status words carry 30-bit counts
 constexpr uint32_t DEFAULT_SPIN_LIMIT = 1u << 20;
 constexpr uint64_t CHUNK_RECORDS = 1u << 16;  // staging ring piece (16.25 MB of 248-byte records)
+constexpr uint64_t DIRECT_COPY_MIN = 1u << 18;  // bytes from which a chunk is copied from the caller's memory itself
 
 template <typename T>
 int dalloc(T** p, size_t count) {
@@ -148,6 +149,7 @@ struct Staging {
     float* pinned[2] = {nullptr, nullptr};
     float* dev[2] = {nullptr, nullptr};
     cudaEvent_t ev[2] = {nullptr, nullptr};
+    cudaStream_t copy = nullptr;  // idle whenever no load is running
     int next = 0;
 };
 
@@ -173,5 +175,7 @@ struct spl_scene {
             stg.pinned[i] = nullptr;
             stg.ev[i] = nullptr;
         }
+        if (stg.copy) cudaStreamDestroy(stg.copy);
+        stg.copy = nullptr;
     }
 };
