@@ -131,26 +131,35 @@ __device__ __forceinline__ uint32_t lookback_single(const uint64_t* status, uint
     return excl;
 }
 
-// Per-thread look-back for one digit of a onesweep pass (status has 256 words per tile).
+// Per-thread look-back for one digit of a onesweep pass (status has 256 words per tile): eight predecessors' words
+// in flight at a time, nearest first, so that a tile whose predecessors have published but not yet looked back, as
+// all of a first wave have, sums them in a few L2 round trips and not in one after another.
 __device__ __forceinline__ uint32_t lookback_digit(const uint64_t* status, uint32_t tile, uint32_t digit,
                                                    uint32_t epoch, uint32_t spin_limit, uint32_t* err) {
-    uint32_t excl = 0;
-    int64_t p = (int64_t)tile - 1;
-    while (p >= 0) {
-        uint64_t s;
-        uint32_t spins = 0;
-        for (;;) {
-            s = lb_load(status + (size_t)p * 256u + digit);
-            if ((uint32_t)(s >> 32) == epoch && ((uint32_t)s & (LB_AGG | LB_INC)) != 0) break;
-            if (++spins > spin_limit) {
-                atomicOr(err, SPL_DEV_ERR_LOOKBACK);
-                return excl;
+    constexpr uint32_t WORDS = 8;
+    uint32_t excl = 0, end = tile;  // tiles before `end` are still to be added
+    while (end > 0u) {
+        const uint32_t m = min(end, WORDS);
+        uint64_t v[WORDS];
+#pragma unroll
+        for (uint32_t j = 0; j < WORDS; ++j)
+            v[j] = j < m ? lb_load(status + (size_t)(end - 1u - j) * 256u + digit) : 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < WORDS; ++j) {
+            if (j >= m) break;
+            uint32_t spins = 0;
+            while ((uint32_t)(v[j] >> 32) != epoch || ((uint32_t)v[j] & (LB_AGG | LB_INC)) == 0u) {
+                if (++spins > spin_limit) {
+                    atomicOr(err, SPL_DEV_ERR_LOOKBACK);
+                    return excl;
+                }
+                if (spins > 16u) __nanosleep(64);
+                v[j] = lb_load(status + (size_t)(end - 1u - j) * 256u + digit);
             }
-            if (spins > 16) __nanosleep(64);
+            excl += (uint32_t)v[j] & LB_VAL;
+            if ((uint32_t)v[j] & LB_INC) return excl;
         }
-        excl += (uint32_t)s & LB_VAL;
-        if ((uint32_t)s & LB_INC) break;
-        --p;
+        end -= m;
     }
     return excl;
 }
