@@ -104,9 +104,11 @@ __global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restr
     float T = 1.0f, Ca[3] = {0.0f, 0.0f, 0.0f};
     const float alpha_min = 1.0f / 255.0f;
     for (uint32_t b = rg.x; b < rg.y; b += RASTER_BATCH) {
-        const uint32_t i = b + tid;
+        const uint32_t i = b + tid, n_left = rg.y - b, slots = listed_slots(n_left);
+        if (tid < slots) {
 #pragma unroll
-        for (int sw = 0; sw < 8; ++sw) s_pm[sw][tid] = 0u;
+            for (int sw = 0; sw < 8; ++sw) s_pm[sw][tid] = 0u;
+        }
         if (i < rg.y) {
             const uint32_t rs = __ldg(pair_vals + i);
             const float4* r = rec + (size_t)rs * 4;
@@ -126,7 +128,7 @@ __global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restr
             {
                 uint32_t n[8] = {};
 #pragma unroll 1
-                for (uint32_t c = 0; c < RASTER_BATCH; c += 32u) {
+                for (uint32_t c = 0; c < slots; c += 32u) {
                     const uint32_t m = s_pm[w][c + lane];
                     if (!__any_sync(FULL_MASK, m != 0u)) continue;
 #pragma unroll
@@ -228,7 +230,8 @@ __global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restr
                 }
             }
         }
-        if (__syncthreads_and(done)) break;
+        // no wait for the other warps after the last batch
+        if (n_left <= (uint32_t)RASTER_BATCH || __syncthreads_and(done)) break;
     }
 }
 

@@ -393,6 +393,22 @@ __device__ __forceinline__ void transpose_lane_bits_n(uint32_t* x, uint32_t lane
     }
 }
 
+// Words c0 ... c0 + N - 1 of the warp's lists (see k_raster), in place.  A group whose records all miss the strip
+// stays zero.
+template <int N>
+__device__ __forceinline__ void list_words(uint32_t (&masks)[RASTER_BATCH], uint32_t c0, uint32_t lane, uint32_t& nz) {
+    uint32_t t[N], any = 0u;
+#pragma unroll
+    for (int c = 0; c < N; ++c) any |= t[c] = masks[(c0 + c) * 32u + lane];
+    if (!__any_sync(FULL_MASK, any != 0u)) return;
+    transpose_lane_bits_n<N>(t, lane);
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+        masks[(c0 + c) * 32u + lane] = t[c];
+        nz |= (t[c] != 0u ? 1u : 0u) << (c0 + c);
+    }
+}
+
 // FAR: a covered pixel's exponent may fall below -87 (axis-aligned squares, or a margin above
 // RASTER_NEAR_MARGIN), where the falloff takes spl_expf's general path.
 template <bool RECT, int BLEND, bool FAR>
@@ -423,8 +439,11 @@ __global__ void __launch_bounds__(256, RASTER_CTAS) k_raster(const uint2* __rest
     const float alpha_min = 1.0f / 255.0f;
     for (uint32_t b = rg.x; b < rg.y; b += RASTER_BATCH) {
         const uint32_t i = b + tid, slot = RASTER_BATCH - 1u - tid;
+        const uint32_t n = rg.y - b;  // records from here on; the batch has 256 of them at most
+        if (tid < listed_slots(n)) {
 #pragma unroll
-        for (int sw = 0; sw < 8; ++sw) s_pm[sw][slot] = 0u;
+            for (int sw = 0; sw < 8; ++sw) s_pm[sw][slot] = 0u;
+        }
         if (i < rg.y) {
             const uint32_t rs = __ldg(pair_vals + i);
             const float4* r = rec + (size_t)rs * 4;
@@ -440,20 +459,13 @@ __global__ void __launch_bounds__(256, RASTER_CTAS) k_raster(const uint2* __rest
             // Per-pixel lists of the batch: the strip's lane masks of slots 32c + l, transposed so that lane p
             // holds word c of pixel p's list (bit i: slot 32c + i); bit c of `nz` marks a non-empty word.
             uint32_t nz = 0u;
-#pragma unroll
-            for (int c0 = 0; c0 < RASTER_WORDS; c0 += 4) {
-                uint32_t t[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) t[c] = s_pm[w][(c0 + c) * 32 + lane];
-                // a group whose 128 records miss the strip stays zero
-                if (__any_sync(FULL_MASK, ((t[0] | t[1]) | (t[2] | t[3])) != 0u)) {
-                    transpose_lane_bits_n<4>(t, lane);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        s_pm[w][(c0 + c) * 32 + lane] = t[c];
-                        nz |= (t[c] != 0u ? 1u : 0u) << (c0 + c);
-                    }
-                }
+            if (n <= 32u) {
+                list_words<1>(s_pm[w], 7u, lane, nz);
+            } else if (n <= 64u) {
+                list_words<2>(s_pm[w], 6u, lane, nz);
+            } else {
+                if (n > 128u) list_words<4>(s_pm[w], 0u, lane, nz);
+                list_words<4>(s_pm[w], 4u, lane, nz);
             }
             // Walk the 32 lists at once across the whole batch: in every iteration each pixel takes its
             // next record.  The warp leaves once every pixel is finished or has walked its list.
@@ -503,7 +515,8 @@ __global__ void __launch_bounds__(256, RASTER_CTAS) k_raster(const uint2* __rest
             }
             warp_done = __all_sync(FULL_MASK, done);
         }
-        if (__syncthreads_and(done)) break;
+        // no wait for the other warps after the last batch
+        if (n <= (uint32_t)RASTER_BATCH || __syncthreads_and(done)) break;
     }
     if (inside) {
         const size_t pix = (size_t)py * (size_t)W + (size_t)px;
