@@ -383,8 +383,17 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
     launch_frame_begin(r->fc, r->epoch, u, r->d_u, sv, r->d_sv, st);
     launch_cull_key(mode, !coop, N, r->d_sv, r->d_u, r->fc, r->epoch, r->st_cull, r->keys_a, r->idx, sl, st);
     r->mark(1, st);
-    launch_preprocess((int)cfg.spherical_harmonics_order, cfg.use_covariance_for_scale != 0,
-                      cfg.use_unaligned_rectangles != 0, r->d_sv, r->d_u, r->idx, r->fc, r->rec, r->boxes, N, st);
+    // The vertex stage and the depth sort both take what the cull kernel leaves.  The cooperative sort goes first and the
+    // vertex stage starts beside it, once all of the sort's CTAs run; while the stages are timed, one after the other.
+    // A short sort is a chain of round trips on a part of the SMs, a long one fills them: frames of 2k splats 35.6 -> 31.1
+    // us, 100k 91.7 -> 87.6, 350k 103.4 -> 95.7, 1M (199k visible) 138.0 -> 121.7, but 6M 877 -> 882 us; a training step
+    // 2797 -> 2688 us.  A second branch of the frame graph instead: 2k 30.1 us, 100k 94.2 us, 1M 3 us faster, 6M 887 us.
+    const bool beside = coop && mode != DS_NONE && N > 0 && N <= BESIDE_MAX && !r->profiling;
+    const auto vertex_stage = [&] {
+        launch_preprocess((int)cfg.spherical_harmonics_order, cfg.use_covariance_for_scale != 0,
+                          cfg.use_unaligned_rectangles != 0, r->d_sv, r->d_u, r->idx, r->fc, r->rec, r->boxes, N, beside, st);
+    };
+    if (!beside) vertex_stage();
     r->mark(2, st);
     const uint32_t* order = nullptr;
     if (mode != DS_NONE && N > 0) {
@@ -392,7 +401,8 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
         if (coop) {
             const SortBuffers io{r->keys_a, nullptr, {r->keys_a, r->keys_b}, {r->vals_a, r->vals_b}, r->keys_a, r->vals_a};
             CU(launch_sort_coop(io, &r->fc->visible, N, 4, 0, r->coop_table, r->epoch, &r->fc->barrier[0].v, sl,
-                                &r->fc->err, st));
+                                &r->fc->err, beside, st));
+            if (beside) vertex_stage();
         } else {
             // digit histograms from the cull kernel; one launch per pass
             uint32_t *src_k = r->keys_a, *dst_k = r->keys_b, *dst_v = r->vals_b;
@@ -422,7 +432,7 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
         const SortBuffers io{r->pk_a, r->pv_a, {r->pk_a, r->pk_b}, {r->pv_a, r->pv_b}, (passes & 1) ? r->pk_b : r->pk_a,
                              (passes & 1) ? r->pv_b : r->pv_a};
         CU(launch_sort_coop(io, &r->fc->pairs, (uint32_t)r->pair_cap, passes, 0, r->coop_table + sort_coop_table_words(),
-                            r->epoch, &r->fc->barrier[1].v, sl, &r->fc->err, st));
+                            r->epoch, &r->fc->barrier[1].v, sl, &r->fc->err, false, st));
     } else {
         // tile-id histograms from the binning kernel
         uint32_t *ak = r->pk_a, *av = r->pv_a, *bk = r->pk_b, *bv = r->pv_b;
@@ -735,7 +745,7 @@ int spl_sort_pairs(spl_renderer* r, const uint32_t* keys_in, const uint32_t* val
         io.vals_out = io.vals[passes & 1];
     }
     CU(launch_sort_coop(io, &r->fc_sort->visible, (uint32_t)count, passes, 0, r->coop_table, r->epoch,
-                        &r->fc_sort->barrier[0].v, r->spin_limit, &r->fc_sort->err, st));
+                        &r->fc_sort->barrier[0].v, r->spin_limit, &r->fc_sort->err, false, st));
     if (!write) {
         CU(cudaMemcpyAsync(keys_out, io.keys_out, bytes, cudaMemcpyDeviceToDevice, st));
         CU(cudaMemcpyAsync(values_out, io.vals_out, bytes, cudaMemcpyDeviceToDevice, st));

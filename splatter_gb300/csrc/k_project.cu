@@ -247,12 +247,12 @@ __global__ void __launch_bounds__(PreShape<SHO, STAGED>::WARPS * 32, PreShape<SH
                                                     const Uniforms* __restrict__ d_u,
                                                     const uint32_t* __restrict__ idx,
                                                     const FrameCounters* __restrict__ fc, float4* __restrict__ rec,
-                                                    uint2* __restrict__ boxes) {
+                                                    uint2* __restrict__ boxes, bool beside) {
     constexpr int NV = PreShape<SHO, STAGED>::NV, STRIDE = PreShape<SHO, STAGED>::STRIDE;
     __shared__ float4 s_sh[PreShape<SHO, STAGED>::WARPS][STAGED ? 32 * STRIDE : 1];
     __shared__ Uniforms s_u;
     __shared__ SceneView s_sv;
-    frame_step(d_sv, d_u, idx, fc);
+    if (!beside) frame_step(d_sv, d_u, idx, fc);
     stage_frame(d_u, s_u, d_sv, s_sv);
     __syncthreads();
     const Uniforms& u = s_u;
@@ -345,34 +345,37 @@ __global__ void __launch_bounds__(PreShape<SHO, STAGED>::WARPS * 32, PreShape<SH
             boxes[slot] = make_uint2(lo, hi);  // compact copy for the binning kernel
         }
     }
+    // This kernel's end is the next one's sign that both are done: one block waits for the kernel before.
+    if (beside && blockIdx.x == 0) frame_step();
 }
 
 template <int SHO, bool COV, bool RECT, bool STAGED>
 static void launch_pre3(const SceneView* s, const Uniforms* u, const uint32_t* idx, const FrameCounters* fc, float4* rec,
-                        uint2* boxes, uint32_t max_n, cudaStream_t st) {
+                        uint2* boxes, uint32_t max_n, bool beside, cudaStream_t st) {
     constexpr uint32_t threads = PreShape<SHO, STAGED>::WARPS * 32;
     // grid stride beyond 4096 threads per SM
     const uint32_t blocks = (max_n + threads - 1) / threads, cap = device_sm_count() * (4096u / threads);
-    launch_after(k_preprocess<SHO, COV, RECT, STAGED>, blocks < cap ? blocks : cap, threads, st, s, u, idx, fc, rec, boxes);
+    launch_after(k_preprocess<SHO, COV, RECT, STAGED>, blocks < cap ? blocks : cap, threads, st, s, u, idx, fc, rec, boxes,
+                 beside);
 }
 template <int SHO>
 static void launch_pre(bool cov, bool rect, const SceneView* s, const Uniforms* u, const uint32_t* idx,
-                       const FrameCounters* fc, float4* rec, uint2* boxes, uint32_t max_n, cudaStream_t st) {
+                       const FrameCounters* fc, float4* rec, uint2* boxes, uint32_t max_n, bool beside, cudaStream_t st) {
     constexpr bool CAN_STAGE = SHO > 0;
     const bool staged = CAN_STAGE && max_n >= PRE_STAGED_MIN;
     auto run = cov ? (rect ? (staged ? launch_pre3<SHO, true, true, CAN_STAGE> : launch_pre3<SHO, true, true, false>)
                            : (staged ? launch_pre3<SHO, true, false, CAN_STAGE> : launch_pre3<SHO, true, false, false>))
                    : (rect ? (staged ? launch_pre3<SHO, false, true, CAN_STAGE> : launch_pre3<SHO, false, true, false>)
                            : (staged ? launch_pre3<SHO, false, false, CAN_STAGE> : launch_pre3<SHO, false, false, false>));
-    run(s, u, idx, fc, rec, boxes, max_n, st);
+    run(s, u, idx, fc, rec, boxes, max_n, beside, st);
 }
 
 void launch_preprocess(int sh_order, bool covariance, bool rect, const SceneView* s, const Uniforms* u,
                        const uint32_t* idx, const FrameCounters* fc, float4* rec, uint2* boxes, uint32_t max_n,
-                       cudaStream_t st) {
+                       bool beside, cudaStream_t st) {
     if (max_n == 0) return;
     auto run = sh_order == 0 ? launch_pre<0> : (sh_order == 1 ? launch_pre<1> : (sh_order == 2 ? launch_pre<2> : launch_pre<3>));
-    run(covariance, rect, s, u, idx, fc, rec, boxes, max_n, st);
+    run(covariance, rect, s, u, idx, fc, rec, boxes, max_n, beside, st);
 }
 
 // ------------------------------------------------------------------------------------------------

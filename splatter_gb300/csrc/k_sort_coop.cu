@@ -42,6 +42,10 @@ constexpr int CS_MIN_SEG = CS_THREADS * 4;    // shortest segment of a sort of s
 constexpr int CS_GROUP = 16;                  // CTAs of a group in the exchange of counts
 constexpr int CS_DIRECT = 32;                 // up to this many CTAs exchange counts without groups
 constexpr int CS_MAX_GRID = 512;
+// Keys up to which the sort leaves room on the SMs for a kernel beside it: its CTAs have 32 K registers each, and
+// one of two on an SM leaves (622 k keys) or ends early (a little above).  With 966 k keys a frame of 1M splats takes
+// 331 us with the vertex stage beside the sort and 324 us without, with 799 k 253.7 and 256.0 us.
+constexpr uint32_t CS_START_MAX = 3u << 18;
 static_assert(CS_THREADS == 512 && CS_WARPS == 16, "the sub-tile scan maps digit t / 2 and 8 warps to thread t, "
                                                    "the exchange digit t & 255 and half of the words");
 
@@ -436,13 +440,14 @@ __device__ __forceinline__ void long_pass(CoopSmem& sm, const CountTable& t, con
 // last pass's buffers are written.
 __global__ void __launch_bounds__(CS_THREADS, 2)
     k_sort_coop(SortBuffers io, const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0, uint64_t* table,
-                const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit, uint32_t* err) {
+                const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit, uint32_t* err, bool start_dependent) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CoopSmem& sm = *reinterpret_cast<CoopSmem*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
     const uint32_t c = blockIdx.x;
     frame_step(n_ptr, epoch_word);
     const uint32_t n = min(*n_ptr, n_cap);
+    if (start_dependent && n <= CS_START_MAX) start_next();
     // Contiguous segments, 256-aligned: up to one sub-tile of keys is one CTA's work, more are spread over
     // the grid in segments of at least CS_MIN_SEG.  The live count is read on the device (a captured graph
     // replays with any count up to n_cap), so the grid is sized for n_cap; CTAs past the last segment
@@ -528,13 +533,14 @@ size_t sort_coop_table_words() { return (size_t)(CS_MAX_GRID + CS_MAX_GRID / CS_
 
 cudaError_t launch_sort_coop(const SortBuffers& io, const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0,
                              uint64_t* table, const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit,
-                             uint32_t* err, cudaStream_t st) {
+                             uint32_t* err, bool start_dependent, cudaStream_t st) {
     if (n_cap == 0 || passes == 0) return cudaSuccess;
     int grid = sort_coop_grid();
     const uint32_t want = (n_cap + CS_MIN_SEG - 1) / CS_MIN_SEG;
     if ((uint32_t)grid > want) grid = (int)want;
     if (grid < 1) grid = 1;
-    void* args[] = {(void*)&io, (void*)&n_ptr, &n_cap, &passes, &shift0, &table, (void*)&epoch_word, &bar, &spin_limit, &err};
+    void* args[] = {(void*)&io, (void*)&n_ptr, &n_cap, &passes, &shift0, &table, (void*)&epoch_word, &bar, &spin_limit, &err,
+                    &start_dependent};
     return cudaLaunchCooperativeKernel((const void*)k_sort_coop, dim3(grid), dim3(CS_THREADS), args,
                                        sizeof(CoopSmem), st);
 }

@@ -37,6 +37,7 @@ inline int fail(int code, const char* fmt, ...) {
 constexpr uint64_t MAX_COUNT = (1ull << 30) - 1;  // look-back status words carry 30-bit counts
 constexpr uint32_t DEFAULT_SPIN_LIMIT = 1u << 20;
 constexpr uint64_t CHUNK_RECORDS = 1u << 16;  // staging ring piece (16.25 MB of 248-byte records)
+constexpr uint32_t BESIDE_MAX = 1u << 20;  // splats up to which the vertex stage is launched beside the depth sort
 constexpr uint64_t DIRECT_COPY_MIN = 1u << 18;  // bytes from which a chunk is copied from the caller's memory itself
 
 template <typename T>

@@ -93,8 +93,10 @@ constexpr int RASTER_OUT_ARG = 10;                // index of the raster kernel'
 void launch_cull_key(int mode, bool hist, uint32_t grid_n, const SceneView* d_sv, const Uniforms* d_u,
                      FrameCounters* fc, const uint32_t* epoch_word, uint64_t* status, uint32_t* keys_out,
                      uint32_t* idx_out, uint32_t spin_limit, cudaStream_t st);
+// beside: it follows a kernel that starts it early, needs nothing from it and started after all that it does need was
+// complete (the depth sort, after the cull kernel); it runs beside that kernel and does not end before it.
 void launch_preprocess(int sh_order, bool covariance, bool rect, const SceneView* d_sv, const Uniforms* d_u,
-                       const uint32_t* idx, const FrameCounters* fc, float4* rec, uint2* boxes, uint32_t max_n,
+                       const uint32_t* idx, const FrameCounters* fc, float4* rec, uint2* boxes, uint32_t max_n, bool beside,
                        cudaStream_t st);
 // One LSD onesweep pass over 8 bits at `shift`.  n = min(*n_ptr, n_cap).  vals_in == nullptr means
 // values are the input positions (0, 1, 2, ...).
@@ -129,7 +131,8 @@ void launch_gather_entries(const uint32_t* keys, const uint32_t* slots, const ui
 // keys[0], vals[0], the output the buffer of its pass; with more than one pass the input may overlap the output.
 // keys_in is 16-byte aligned.  table: sort_coop_table_words() words of its own for each
 // sort of a frame, zero at first and never cleared (the words carry *epoch_word, never 0 and another one at
-// each launch); *bar (the grid barrier's arrival count) must be zero when the launch starts.
+// each launch); *bar (the grid barrier's arrival count) must be zero when the launch starts.  start_dependent: the next
+// kernel of the stream may start as soon as all CTAs run (see launch_preprocess).
 struct SortBuffers {
     const uint32_t *keys_in, *vals_in;
     uint32_t *keys[2], *vals[2];
@@ -137,7 +140,7 @@ struct SortBuffers {
 };
 cudaError_t launch_sort_coop(const SortBuffers& io, const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0,
                              uint64_t* table, const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit,
-                             uint32_t* err, cudaStream_t st);
+                             uint32_t* err, bool start_dependent, cudaStream_t st);
 size_t sort_coop_table_words();
 int sort_coop_grid();
 // The loader's activations of raw parameters and their backward (k_activate.cu).
