@@ -319,8 +319,9 @@ int spl_renderer_create(const spl_config* cfg, spl_renderer** out) {
     TRY(dalloc(&r->epoch, 1));
     TRY(dalloc(&r->d_u, 1));
     TRY(dalloc(&r->d_sv, 1));
-    TRY(dalloc(&r->coop_table, 2 * sort_coop_table_words()));
-    (void)sort_coop_grid();  // its one-time occupancy query, outside any stream capture
+    // (the words' count asks the sort's occupancy once, outside any stream capture)
+    const size_t table_words = sort_coop_table_words(r->max_n) + sort_coop_table_words(r->pair_cap);
+    TRY(dalloc(&r->coop_table, table_words));
 #undef TRY
     cudaError_t e = cudaSuccess;
     // status words start at epoch 0, which no frame uses
@@ -329,7 +330,7 @@ int spl_renderer_create(const spl_config* cfg, spl_renderer** out) {
     if (e == cudaSuccess) e = cudaMemset(r->fc, 0, sizeof(FrameCounters));
     if (e == cudaSuccess) e = cudaMemset(r->fc_sort, 0, sizeof(FrameCounters));
     if (e == cudaSuccess)
-        e = cudaMemset(r->coop_table, 0, 2 * sort_coop_table_words() * 8);
+        e = cudaMemset(r->coop_table, 0, table_words * 8);
     if (e == cudaSuccess) e = cudaMemset(r->epoch, 0, 4);
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&r->host_fc), sizeof(FrameCounters));
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -431,7 +432,7 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
     if (coop) {
         const SortBuffers io{r->pk_a, r->pv_a, {r->pk_a, r->pk_b}, {r->pv_a, r->pv_b}, (passes & 1) ? r->pk_b : r->pk_a,
                              (passes & 1) ? r->pv_b : r->pv_a};
-        CU(launch_sort_coop(io, &r->fc->pairs, (uint32_t)r->pair_cap, passes, 0, r->coop_table + sort_coop_table_words(),
+        CU(launch_sort_coop(io, &r->fc->pairs, (uint32_t)r->pair_cap, passes, 0, r->coop_table + sort_coop_table_words(r->max_n),
                             r->epoch, &r->fc->barrier[1].v, sl, &r->fc->err, false, st));
     } else {
         // tile-id histograms from the binning kernel

@@ -69,7 +69,7 @@ struct CountTable {
     uint64_t* rows;    // [CTA][256], then [group][256]
     uint32_t epoch, pass, spin_limit;
     uint32_t* err;
-    __device__ __forceinline__ uint64_t* group(uint32_t g) const { return rows + ((size_t)CS_MAX_GRID + g) * 256; }
+    __device__ __forceinline__ uint64_t* group(uint32_t g) const { return rows + ((size_t)gridDim.x + g) * 256; }
     __device__ __forceinline__ void publish(uint64_t* p, uint32_t count) const { lb_store(p, count_word(epoch, pass, count)); }
     // Adds the counts of rows first, first + 2, ... < end (word d of each) to tot, those before `mine` to pre;
     // eight loads in flight.  A word that does not become valid in time counts as zero (the error bit is set).
@@ -529,19 +529,24 @@ int sort_coop_grid() {
     return g_cs_grid;
 }
 
-size_t sort_coop_table_words() { return (size_t)(CS_MAX_GRID + CS_MAX_GRID / CS_GROUP) * 256; }
+// CTAs launched for at most n_cap keys.
+static uint32_t coop_grid_for(uint64_t n_cap) {
+    const uint64_t grid = (uint64_t)sort_coop_grid(), want = (n_cap + CS_MIN_SEG - 1) / CS_MIN_SEG;
+    return (uint32_t)(want < 1 ? 1 : (want < grid ? want : grid));
+}
+
+size_t sort_coop_table_words(uint64_t n_cap) {
+    const size_t grid = coop_grid_for(n_cap);
+    return (grid + (grid + CS_GROUP - 1) / CS_GROUP) * 256;
+}
 
 cudaError_t launch_sort_coop(const SortBuffers& io, const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0,
                              uint64_t* table, const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit,
                              uint32_t* err, bool start_dependent, cudaStream_t st) {
     if (n_cap == 0 || passes == 0) return cudaSuccess;
-    int grid = sort_coop_grid();
-    const uint32_t want = (n_cap + CS_MIN_SEG - 1) / CS_MIN_SEG;
-    if ((uint32_t)grid > want) grid = (int)want;
-    if (grid < 1) grid = 1;
     void* args[] = {(void*)&io, (void*)&n_ptr, &n_cap, &passes, &shift0, &table, (void*)&epoch_word, &bar, &spin_limit, &err,
                     &start_dependent};
-    return cudaLaunchCooperativeKernel((const void*)k_sort_coop, dim3(grid), dim3(CS_THREADS), args,
+    return cudaLaunchCooperativeKernel((const void*)k_sort_coop, dim3(coop_grid_for(n_cap)), dim3(CS_THREADS), args,
                                        sizeof(CoopSmem), st);
 }
 

@@ -129,7 +129,7 @@ void launch_gather_entries(const uint32_t* keys, const uint32_t* slots, const ui
 // vals_in (no vals_in: the values are the positions), the last pass writes keys_out and vals_out, and in between
 // pass p writes keys[1], vals[1] (p even) or keys[0], vals[0] (p odd) for the next.  The input may be
 // keys[0], vals[0], the output the buffer of its pass; with more than one pass the input may overlap the output.
-// keys_in is 16-byte aligned.  table: sort_coop_table_words() words of its own for each
+// keys_in is 16-byte aligned.  table: sort_coop_table_words(n_cap) words of its own for each
 // sort of a frame, zero at first and never cleared (the words carry *epoch_word, never 0 and another one at
 // each launch); *bar (the grid barrier's arrival count) must be zero when the launch starts.  start_dependent: the next
 // kernel of the stream may start as soon as all CTAs run (see launch_preprocess).
@@ -141,7 +141,7 @@ struct SortBuffers {
 cudaError_t launch_sort_coop(const SortBuffers& io, const uint32_t* n_ptr, uint32_t n_cap, int passes, int shift0,
                              uint64_t* table, const uint32_t* epoch_word, uint32_t* bar, uint32_t spin_limit,
                              uint32_t* err, bool start_dependent, cudaStream_t st);
-size_t sort_coop_table_words();
+size_t sort_coop_table_words(uint64_t n_cap);
 int sort_coop_grid();
 // The loader's activations of raw parameters and their backward (k_activate.cu).
 void launch_activate(uint32_t n, const float* means, const float* quats, const float* logs, const float* logits,
