@@ -23,9 +23,12 @@ constexpr uint32_t FULL_MASK = 0xFFFFFFFFu;
 // takes what such loads read for unchanging and might read it before the wait otherwise.
 // Frames of 2k splats 44.6 -> 38.3 us, of 100k 101.4 -> 99.4 us, of 1M 188.3 -> 187.1 us, of 6M the same; the backward of
 // eight views of 1M splats 1829 -> 1762 us.
-// start_next is called by the kernels of one block only (frame start, tile order: thumbnails and 1M splats gain
+// start_next is called by the kernels of one block (frame start, tile order: thumbnails and 1M splats gain
 // 0.4 and 1.3 us); called by all, the next kernel's waiting blocks take room from the last wave (100k splats
 // 105.5 us, 6M +10 us), and the cooperative sorts stay plain dependents for the same reason.
+// The cooperative depth sort calls it too, when all that the vertex stage reads is complete (the sort itself starts
+// after the cull kernel has ended): the vertex stage then runs beside the sort without a wait at its start, and its
+// first block waits at its end, so that the kernels after it, which wait for it alone, find both complete.
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
