@@ -12,7 +12,7 @@
 //     dL/ds_c  = dL/dC_c * T_i
 //     dL/dsa   = -(dL/dC . S + dL/dT * T_final) / (1 - sa)
 // and the chain through sat(), the falloff and tc = A (X, Y) + B gives per-splat gradients of the
-// record (A00, A01, B0, A10, A11, B1, a, r, g, b), reduced over each 2x2-pixel group before one
+// record (A00, A01, B0, A10, A11, B1, a, r, g, b), reduced over each 4x2-pixel group before one
 // set of global float atomics per (splat, group).  A is accumulated against pixel offsets from the
 // centre of the splat's pixel box and B at that centre (well conditioned; see vertex_vjp_t).
 //
@@ -35,35 +35,47 @@ __global__ void k_zero_grad_rec(float* grad_rec, const FrameCounters* fc, uint32
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) grad_rec[i] = 0.0f;
 }
 
-// Sums 10 values over the 4 lanes of a lane group in two exchange steps that halve the values each lane carries:
-// lane li = 2 h2 + h1 gets the sums of values k0 = 5 h2 + 3 h1 on, three of them (h1 = 0) or two.
-__device__ __forceinline__ uint32_t reduce10_over4(const float* g, uint32_t li, float (&v)[3]) {
-    const bool h2 = (li & 2u) != 0u, h1 = (li & 1u) != 0u;
-    float a[5];
+// Sums 10 values over the 8 lanes of a lane group (lane index li = lane & 7) in three exchange steps that halve the
+// values each lane carries: afterwards lane li holds the sum of value k0 in v0 and, for li = 0 and 4, of k0 + 1 in v1.
+__device__ __forceinline__ uint32_t reduce10_over8(const float* g, uint32_t li, float& v0, float& v1) {
+    const bool h4 = (li & 4u) != 0u, h2 = (li & 2u) != 0u, h1 = (li & 1u) != 0u;
+    float a[5], b[3];
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {  // keep values 5..9 (h2) or 0..4
-        const float send = h2 ? g[i] : g[i + 5], keep = h2 ? g[i + 5] : g[i];
-        a[i] = keep + __shfl_xor_sync(FULL_MASK, send, 2);
+    for (int i = 0; i < 5; ++i) {  // keep values 5..9 (h4) or 0..4
+        const float send = h4 ? g[i] : g[i + 5], keep = h4 ? g[i + 5] : g[i];
+        a[i] = keep + __shfl_xor_sync(FULL_MASK, send, 4);
     }
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {  // keep a[3..4] (h1) or a[0..2]
+    for (int i = 0; i < 3; ++i) {  // keep a[3..4] (h2) or a[0..2]
         const float hi = i < 2 ? a[i + 3] : 0.0f;
-        const float send = h1 ? a[i] : hi, keep = h1 ? hi : a[i];
-        v[i] = keep + __shfl_xor_sync(FULL_MASK, send, 1);
+        const float send = h2 ? a[i] : hi, keep = h2 ? hi : a[i];
+        b[i] = keep + __shfl_xor_sync(FULL_MASK, send, 2);
     }
-    return (h2 ? 5u : 0u) + (h1 ? 3u : 0u);
+    // h2 lanes carry two values (b0, b1): keep b1 (h1) or b0; the others three: keep b2 (h1) or b0, b1
+    const float send0 = h1 ? b[0] : (h2 ? b[1] : b[2]);
+    const float keep0 = h1 ? (h2 ? b[1] : b[2]) : b[0];
+    const float send1 = (h1 && !h2) ? b[1] : 0.0f;
+    const float keep1 = (!h1 && !h2) ? b[1] : 0.0f;
+    v0 = keep0 + __shfl_xor_sync(FULL_MASK, send0, 1);
+    v1 = keep1 + __shfl_xor_sync(FULL_MASK, send1, 1);
+    return (h4 ? 5u : 0u) + (h2 ? (h1 ? 4u : 3u) : (h1 ? 2u : 0u));
 }
 
-// One CTA per tile, its warps as in k_raster (strips of two rows), a warp's lanes in eight groups of 2x2 pixels.
+// One CTA per tile, its warps as in k_raster (strips of two rows), a warp's lanes in four groups of 4x2 pixels.
 // A group walks its own list of the batch's records, those whose row masks (mask_rows) touch one of its pixels,
-// all four lanes on the same record, so that the record's ten gradients are summed over the group before they
-// are added to grad_rec.  The lists are record indices in shared memory: eight ballots per 32 records give every
+// all eight lanes on the same record, so that the record's ten gradients are summed over the group before they
+// are added to grad_rec.  The lists are record indices in shared memory: four ballots per 32 records give every
 // (record, group) its place, and the walk has no list bookkeeping but a counter.
-// Bound by instruction issue (70% of the slots at 32 warps per SM, DRAM 7%): what counts is the number of walk
-// iterations, i.e. how well the lists fit, and what one costs.  Per view of 1M splats at 1024x1024, 8 views:
-// groups of 4x2 pixels listed by their boxes and walked in lockstep over 32 records 167 us; lists from the row
-// masks, walked over the whole batch, 134 us; groups of 2x2 pixels (fewer idle lanes, two exchange steps instead
-// of three, more atomics) 116 us; lists as record indices instead of bit words 111 us.
+// Bound by instruction issue (DRAM 7%): what counts is the number of walk iterations, i.e. how well the lists fit, and
+// what one costs.  A training step of eight views of 1M splats at 1024x1024, per view: groups listed by their boxes and
+// walked in lockstep over 32 records 167 us; lists from the row masks, walked over the whole batch as bit words, 134 us;
+// as record indices 125 us (106 us as a launch alone).
+// Groups of 2x2 pixels take 111 us (99 us), with fewer idle lanes, but twice as many additions to grad_rec: one after
+// another to one float, their error grows with the square root of their number, 2.31e-7 of a sum for 1.72e-7
+// (root mean square of colour gradients over some 130 groups of 4x2), and the vertex stage's sweep passes a thousandfold
+// of it on to the rotations of nearly round splats (1.3e-3 between two sums of a step instead of 5.6e-4 at worst).
+// Sums in double of either group have neither, but cost more than the smaller groups save (a step 2,931 us with 4x2 and
+// float, 3,030 with 2x2 and double, 3,087 with 4x2 and double) and twice the scratch.
 template <bool RECT, bool FAR>
 __global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restrict__ ranges,
                                                          const uint4* __restrict__ tile_order,
@@ -77,9 +89,9 @@ __global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restr
     __shared__ float4 s_a[RASTER_BATCH], s_b[RASTER_BATCH], s_c[RASTER_BATCH];
     __shared__ float4 s_q3[RECT ? 1 : RASTER_BATCH];
     __shared__ uint32_t s_row[RASTER_BATCH], s_pm[8][RASTER_BATCH];  // the record's row of grad_rec; its row masks
-    __shared__ uint8_t s_list[8][8][RASTER_BATCH];                   // [warp][group]
+    __shared__ uint8_t s_list[8][4][RASTER_BATCH];                   // [warp][group]
     const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5, lt = lanemask_lt();
-    const uint32_t grp = lane >> 2, li = lane & 3u;
+    const uint32_t grp = lane >> 3, li = lane & 7u;
     frame_step(ranges, tile_order, pair_vals, rec, image, grad_image);
     // the forward's most-pairs-first order of this frame's tiles, when it made one
     uint2 rg;
@@ -87,7 +99,7 @@ __global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restr
     ordered_tile(ranges, tile_order, rg, tile);
     const int tx = tile % tiles_x, ty = tile / tiles_x;
     const int wx0 = tx * TILE_PIXELS, ty0 = ty * TILE_PIXELS;
-    const uint32_t col = 2u * grp + (li & 1u), row = li >> 1;
+    const uint32_t col = 4u * grp + (li & 3u), row = li >> 2;
     const int px = wx0 + (int)col, py = ty0 + 2 * (int)w + (int)row;
     const float X = (float)px + 0.5f, Y = (float)py + 0.5f;
     const uint32_t my_pixel = 1u << (16u * row + col);  // in a strip's row mask
@@ -126,21 +138,21 @@ __global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restr
         if (__any_sync(FULL_MASK, !done)) {
             uint32_t count = 0u, longest = 0u;  // entries of this lane's group's list, and of the warp's longest
             {
-                uint32_t n[8] = {};
+                uint32_t n[4] = {};
 #pragma unroll 1
                 for (uint32_t c = 0; c < slots; c += 32u) {
                     const uint32_t m = s_pm[w][c + lane];
                     if (!__any_sync(FULL_MASK, m != 0u)) continue;
 #pragma unroll
-                    for (uint32_t q = 0; q < 8u; ++q) {
-                        const bool hit = (m & (0x00030003u << (2u * q))) != 0u;
+                    for (uint32_t q = 0; q < 4u; ++q) {
+                        const bool hit = (m & (0x000F000Fu << (4u * q))) != 0u;
                         const uint32_t hits = __ballot_sync(FULL_MASK, hit);
                         if (hit) s_list[w][q][n[q] + __popc(hits & lt)] = (uint8_t)(c + lane);
                         n[q] += __popc(hits);
                     }
                 }
 #pragma unroll
-                for (uint32_t q = 0; q < 8u; ++q) {
+                for (uint32_t q = 0; q < 4u; ++q) {
                     count = grp == q ? n[q] : count;
                     longest = max(longest, n[q]);
                 }
@@ -219,13 +231,12 @@ __global__ void __launch_bounds__(256, 4) k_raster_backward(const uint2* __restr
                 // reduce over the lanes of the group (all hold the same record this iteration)
                 const uint32_t gm = __ballot_sync(FULL_MASK, contrib);
                 if (gm != 0u) {
-                    float v[3];
-                    const uint32_t k0 = reduce10_over4(g, li, v);
-                    if ((gm >> (grp * 4u)) & 0xFu) {
+                    float v0, v1;
+                    const uint32_t k0 = reduce10_over8(g, li, v0, v1);
+                    if ((gm >> (grp * 8u)) & 0xFFu) {
                         float* dst = grad_rec + (size_t)s_row[j] * GR + k0;
-                        atomicAdd(dst, v[0]);
-                        atomicAdd(dst + 1, v[1]);
-                        if (!(li & 1u)) atomicAdd(dst + 2, v[2]);
+                        atomicAdd(dst, v0);
+                        if ((li & 3u) == 0u) atomicAdd(dst + 1, v1);
                     }
                 }
             }
