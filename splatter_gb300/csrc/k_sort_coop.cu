@@ -30,6 +30,8 @@
 // (writes stay in bounds), so a missing CTA can never hang the GPU.  The barrier word counts the
 // launch's arrivals and must be zero when the launch starts (each sort of a frame has its own word in
 // the frame counters, which the frame start zeroes).
+#include <atomic>
+
 #include "spl_device.cuh"
 
 namespace spl {
@@ -514,19 +516,23 @@ __global__ void __launch_bounds__(CS_THREADS, 2)
     }
 }
 
-static int g_cs_grid = 0;
-
+// CTAs of the grid on the current device, asked of each device once: they are what the device holds at a time, and the
+// kernel's shared memory (above the 48 KB that every kernel may have) is allowed device by device.
 int sort_coop_grid() {
-    if (g_cs_grid == 0) {
-        int dev = 0, sms = 0, per = 0;
-        cudaGetDevice(&dev);
+    static std::atomic<int> cache[64];
+    int dev = 0;
+    const bool known = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
+    int grid = known ? cache[dev].load(std::memory_order_relaxed) : 0;
+    if (grid == 0) {
+        int sms = 0, per = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaFuncSetAttribute(k_sort_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CoopSmem));
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sort_coop, CS_THREADS, sizeof(CoopSmem));
-        g_cs_grid = sms * (per > 0 ? per : 1);
-        if (g_cs_grid > CS_MAX_GRID) g_cs_grid = CS_MAX_GRID;
+        grid = sms * (per > 0 ? per : 1);
+        if (grid > CS_MAX_GRID) grid = CS_MAX_GRID;
+        if (known) cache[dev].store(grid, std::memory_order_relaxed);
     }
-    return g_cs_grid;
+    return grid;
 }
 
 // CTAs launched for at most n_cap keys.
