@@ -233,14 +233,14 @@ def load_peaks():
 
 
 # DRAM traffic per unit of the dominant kernel, from one ncu capture of a smaller case of the same
-# workload (k_raster on 3M splats, 1920x1080, fly-through pose 2: 3,353,969 pairs, 240.6 MB read + 6.4
-# MB written): the reads grow with the pairs, the image write is per launch.  The bench scales it to
-# its own frames by their pair counts.
-TRAFFIC_PER_UNIT = {"raster": {"per_pair": 240.6e6 / 3353969.0, "per_launch": 6.4e6,
+# workload (k_raster on 3M splats, 1920x1080, fly-through pose 2, profiles/frame_3m_1080p.md: 3,353,969 pairs,
+# 241.8 MB read + 7.3 MB written): the reads grow with the pairs, the image write is per launch.  The bench
+# scales it to its own frames by their pair counts.
+TRAFFIC_PER_UNIT = {"raster": {"per_pair": 241.8e6 / 3353969.0, "per_launch": 7.3e6,
                                "source": "ncu capture of k_raster at 3M splats, 1080p (pose 2), scaled by pairs"}}
 # The raster is bound by instruction issue, not HBM: the fraction of issue slots its warps used in the
 # same capture (smsp__issue_active, pct of peak, active), reported beside the HBM figure.
-ISSUE_ACTIVE = {"raster": {"frac": 0.836, "source": "ncu smsp__issue_active of the same k_raster capture"}}
+ISSUE_ACTIVE = {"raster": {"frac": 0.808, "source": "ncu smsp__issue_active of the same k_raster capture"}}
 
 
 def stage_traffic(stage, P):

@@ -175,9 +175,12 @@ SPL_API int spl_parse_file_header(const char* path, uint32_t* header_bytes, uint
 
 /* Scene::load_chunk (scene.rs:216-264) from host memory: `count` records of 62 floats (248 bytes,
  * scene.rs:15-24) for splats [start, start+count) (clamped to the scene, scene.rs:217).  The
- * records are staged through pinned memory and copied with cudaMemcpyAsync; the transform (rotor
- * normalisation, clamped exp of the log-scales, sigmoid opacity, SH copy) runs on the device.  The
- * host buffer may be reused when the call returns; the device work is asynchronous on `stream`. */
+ * transform (rotor normalisation, clamped exp of the log-scales, sigmoid opacity, SH copy) runs on the
+ * device, asynchronously on `stream`; the host buffer has been read when the call returns and may be
+ * reused.  Records of 256 KB or more are copied from the host buffer itself, on a stream of the scene's
+ * own that the call waits for, where the device reads host memory through the host's page tables;
+ * otherwise, and while `stream` is being captured, they are staged through pinned memory and copied on
+ * `stream`. */
 SPL_API int spl_scene_load_chunk(spl_scene* s, const void* records, uint64_t start, uint64_t count, void* stream);
 
 /* Scene::load_chunk reading the records straight from a splat file (seek to header + start*248,
@@ -313,13 +316,15 @@ SPL_API int spl_sort_pairs_no_alloc_status(void* stream, uint32_t* device_error)
 /* ---- diagnostics ----------------------------------------------------------------------------------- */
 /* Stage timing with CUDA events on the launching stream (off by default).  When enabled, each
  * render_frame records events between its stages; spl_renderer_stage_times waits for the last frame
- * and writes SPL_STAGE_COUNT durations in milliseconds, indexed by SPL_STAGE_*.  The stages run one
- * after another on the frame's stream, so they add up to the frame time. */
+ * and writes SPL_STAGE_COUNT durations in milliseconds, indexed by SPL_STAGE_*.  Timed stages run one
+ * after another on the frame's stream, so they add up to the timed frame's time; with stage timing off
+ * a stage's kernels may start before the one before has ended, and frames of up to 2^20 splats run
+ * their vertex stage beside the cooperative depth sort. */
 #define SPL_STAGE_CULL 0       /* frame start, cull + key + ordered compaction */
 #define SPL_STAGE_PREPROCESS 1 /* vertex stage: colour, conic, rectangle records */
 #define SPL_STAGE_DEPTH_SORT 2 /* the stable depth sort of the visible keys (one cooperative launch,
                                   or one onesweep launch per digit pass) */
-#define SPL_STAGE_BIN 3        /* tile-range clear + tile binning */
+#define SPL_STAGE_BIN 3        /* tile binning (and emptying the tiles' ranges) */
 #define SPL_STAGE_PAIR_SORT 4  /* the stable sort of the (tile, splat) pairs by tile id */
 #define SPL_STAGE_RANGES 5     /* per-tile list ranges */
 #define SPL_STAGE_RASTER 6     /* tile order + tile raster + blend */
@@ -327,8 +332,7 @@ SPL_API int spl_sort_pairs_no_alloc_status(void* stream, uint32_t* device_error)
 #define SPL_STAGE_COUNT 8
 SPL_API int spl_renderer_set_profiling(spl_renderer* r, int enable);
 SPL_API int spl_renderer_stage_times(spl_renderer* r, float* milliseconds, int count);
-/* Number of kernel launches (plus memsets) one render_frame issues with this configuration at this
- * viewport. */
+/* Number of kernel launches one render_frame issues with this configuration at this viewport. */
 SPL_API int spl_renderer_launches_per_frame(const spl_renderer* r, uint32_t width, uint32_t height);
 
 /* ---- sort algorithm (extension) -----------------------------------------------------------------

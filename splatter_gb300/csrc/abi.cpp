@@ -387,8 +387,10 @@ static int render_frame_impl(spl_renderer* r, const SceneView& sv, const Uniform
     // The vertex stage and the depth sort both take what the cull kernel leaves.  The cooperative sort goes first and the
     // vertex stage starts beside it, once all of the sort's CTAs run; while the stages are timed, one after the other.
     // A short sort is a chain of round trips on a part of the SMs, a long one fills them: frames of 2k splats 35.6 -> 31.1
-    // us, 100k 91.7 -> 87.6, 350k 103.4 -> 95.7, 1M (199k visible) 138.0 -> 121.7, but 6M 877 -> 882 us; a training step
-    // 2797 -> 2688 us.  A second branch of the frame graph instead: 2k 30.1 us, 100k 94.2 us, 1M 3 us faster, 6M 887 us.
+    // us, 100k 91.7 -> 87.6, 350k 103.4 -> 95.7, 1M (199k visible) 138.0 -> 121.7; a training step 2797 -> 2688 us.  Above
+    // BESIDE_MAX the gain is 1% where a fifth of the splats is visible (1.5M 173.9 -> 171.6 us, 2M 211.2 -> 209.6) and the loss
+    // as much where most are (2M 454.6 -> 459.9, 3M 551.0 -> 554.2, 6M 877 -> 882).  A second branch of the frame graph
+    // instead: 2k 30.1 us, 100k 94.2 us, 1M 3 us faster, 6M 887 us.
     const bool beside = coop && mode != DS_NONE && N > 0 && N <= BESIDE_MAX && !r->profiling;
     const auto vertex_stage = [&] {
         launch_preprocess((int)cfg.spherical_harmonics_order, cfg.use_covariance_for_scale != 0,

@@ -66,7 +66,7 @@ __device__ __forceinline__ uint32_t reduce10_over8(const float* g, uint32_t li, 
 // all eight lanes on the same record, so that the record's ten gradients are summed over the group before they
 // are added to grad_rec.  The lists are record indices in shared memory: four ballots per 32 records give every
 // (record, group) its place, and the walk has no list bookkeeping but a counter.
-// Bound by instruction issue (DRAM 7%): what counts is the number of walk iterations, i.e. how well the lists fit, and
+// Bound by instruction issue (74% of the slots, DRAM 5%): what counts is the number of walk iterations, i.e. how well the lists fit, and
 // what one costs.  A training step of eight views of 1M splats at 1024x1024, per view: groups listed by their boxes and
 // walked in lockstep over 32 records 167 us; lists from the row masks, walked over the whole batch as bit words, 134 us;
 // as record indices 125 us (106 us as a launch alone).

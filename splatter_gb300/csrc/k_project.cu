@@ -76,7 +76,8 @@ __device__ __forceinline__ void stage_frame(const Uniforms* __restrict__ d_u, Un
 // Bound by latency: the ticket and the uniform block, the loads, some 120 instructions per splat, the look-back.
 // 6M splats 66 -> 50 us (look-back words in lines of their own and 256 of them per step: 52 us; tiles of 2048 splats
 // instead of 4096, four CTAs per SM: 50 us, tiles of 1024: 61 us), 1M 26 -> 21 us; frames of up to 2^19 splats,
-// which fit one wave in tiles of 1024, take those: 100k 18 -> 15 us, 350k 19 -> 16 us.
+// which fit one wave in tiles of 1024, take those: 100k 18 -> 15 us, 350k 19 -> 16 us (whole frames of 131k 67.8 -> 66.4 us,
+// 400k 84.8 -> 84.5, 2^19 the same, 700k 103.0 -> 105.0, 1M 121.5 -> 123.6).
 template <int MODE, bool HIST, int PER_LANE>
 __global__ void __launch_bounds__(256, 4) k_cull_key(const SceneView* __restrict__ d_sv, const Uniforms* __restrict__ d_u,
                                                   FrameCounters* fc,
@@ -220,13 +221,14 @@ void launch_cull_key(int mode, bool hist, uint32_t grid_n, const SceneView* d_sv
 // Vertex stage, a warp for 32 visible splats at a time.  STAGED: their SH rows (NV 16-byte pieces of the
 // 192-byte rows) come through shared memory: lane l of load k copies piece (32 k + l) of the warp's 32 NV
 // pieces, so that a load's lanes cover whole rows.  One row per lane instead touches 32 different 128-byte
-// lines with every load, and the L1's line accesses bound the kernel (78% of their peak, 408 per warp of 32
-// splats).  The copies are asynchronous: the shape is computed while they are in flight.  6M splats, SH 3,
-// 4.33M visible: 246 -> 219 us, 91% of the copy bandwidth on 312 bytes per visible splat (seven CTAs of four
-// warps per SM at 72 registers; six 223 us; eight 219 us, but slower than seven below 1M splats; a grid of the
-// resident CTAs alone 228 us).  Where one wave of warps holds all splats the detour only adds latency (frames
-// of 2k, 100k and 350k splats 0.8-1.2 us longer, 1M splats 1.1 us shorter): below PRE_STAGED_MIN splats,
-// and for degree 0, whose rows are one piece, each lane reads its own row.
+// lines with every load, and the L1's line accesses bound the kernel.  The copies are asynchronous: the shape
+// is computed while they are in flight.  6M splats, SH 3, 4.33M visible: 246 -> 219 us, 91% of the copy
+// bandwidth on 312 bytes per visible splat (seven CTAs of four warps per SM at 72 registers; six 223 us; eight
+// 219 us, but slower than seven below 1M splats; a grid of the resident CTAs alone 228 us).  Where one wave of
+// warps holds all splats the detour only adds latency (before the stage ran beside the sort, frames of 2k, 100k
+// and 350k splats 0.8-1.2 us longer; since, with nearly all splats visible, 262k 151.3 -> 152.6 us, 400k 202.3
+// -> 202.1, 2^19 234.4 -> 230.5, 1M 332.8 -> 324.0): below PRE_STAGED_MIN splats, and for degree 0, whose rows
+// are one piece, each lane reads its own row.
 constexpr uint32_t PRE_STAGED_MIN = 1u << 19;
 
 template <int SHO, bool STAGED>

@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(1024) k_tile_order(const uint2* __restrict__ r
 // walked in depth order per pixel, a warp whose pixels are all finished skips the rest, and the CTA stops
 // once every pixel is finished (T == 0 in unorm8 mode, T < 1e-4 in fp32 mode).
 //
-// Bound by instruction issue (3M splats, 1080p: 78% of issue slots, 192 M warp instructions, DRAM 5%), so the
+// Bound by instruction issue (3M splats, 1080p: 81% of issue slots, 194 M warp instructions, DRAM 16%), so the
 // work per list entry and per record is what counts:
 // * lists exact to a pixel row (column interval per row) instead of to a 2x2 block: a walk iteration's lanes
 //   rarely miss the rectangle.  6M splats, 1080p: 400 -> 360 us; 3840x2160: 1,002 -> 924 us;

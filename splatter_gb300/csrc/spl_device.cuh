@@ -17,18 +17,20 @@ constexpr uint32_t FULL_MASK = 0xFFFFFFFFu;
 // ------------------------------------------------------------------------------------------------
 // A frame's kernels, and those of its backward, are launched with programmatic dependence (launch_after): a kernel's blocks may start when
 // every block of the kernel before it has ended or called start_next, instead of after a full launch latency.
-// Every kernel calls frame_step before it touches memory: it waits until the kernel before has ended and its
+// Every kernel but one calls frame_step before it touches memory: it waits until the kernel before has ended and its
 // writes are visible (at once, where a kernel is launched plainly), so a kernel sees all kernels before it
-// complete.  The pointers that it reads through the read-only path are given to frame_step: the compiler
+// complete.  The exception is the vertex stage beside the depth sort (below), which reads only what was complete before
+// that sort began: a kernel between the two, or one more input of the vertex stage that the sort or a kernel between
+// writes, would break it.  The pointers that it reads through the read-only path are given to frame_step: the compiler
 // takes what such loads read for unchanging and might read it before the wait otherwise.
 // Frames of 2k splats 44.6 -> 38.3 us, of 100k 101.4 -> 99.4 us, of 1M 188.3 -> 187.1 us, of 6M the same; the backward of
 // eight views of 1M splats 1829 -> 1762 us.
 // start_next is called by the kernels of one block (frame start, tile order: thumbnails and 1M splats gain
 // 0.4 and 1.3 us); called by all, the next kernel's waiting blocks take room from the last wave (100k splats
 // 105.5 us, 6M +10 us), and the cooperative sorts stay plain dependents for the same reason.
-// The cooperative depth sort calls it too, when all that the vertex stage reads is complete (the sort itself starts
-// after the cull kernel has ended): the vertex stage then runs beside the sort without a wait at its start, and its
-// first block waits at its end, so that the kernels after it, which wait for it alone, find both complete.
+// The cooperative depth sort calls it too, when all that the vertex stage reads is complete (the sort itself is launched
+// plainly and starts after the cull kernel has ended): the vertex stage then runs beside the sort without a wait at its
+// start, and its first block waits at its end, so that the kernels after it, which wait for it alone, find both complete.
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
