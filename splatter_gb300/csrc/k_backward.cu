@@ -73,7 +73,8 @@ __device__ __forceinline__ uint32_t reduce10_over8(const float* g, uint32_t li, 
 // Groups of 2x2 pixels take 111 us (99 us), with fewer idle lanes, but twice as many additions to grad_rec: one after
 // another to one float, their error grows with the square root of their number, 2.31e-7 of a sum for 1.72e-7
 // (root mean square of colour gradients over some 130 groups of 4x2), and the vertex stage's sweep passes a thousandfold
-// of it on to the rotations of nearly round splats (1.3e-3 between two sums of a step instead of 5.6e-4 at worst).
+// of it on to the rotations of nearly round splats (the worst splat of a million against the 4x2 groups in another order,
+// nine in ten of 70 scenes: below 6.0e-4 of its gradient with 2x2, 2.4e-4 with 4x2).
 // Sums in double of either group have neither, but cost more than the smaller groups save (a step 2,931 us with 4x2 and
 // float, 3,030 with 2x2 and double, 3,087 with 4x2 and double) and twice the scratch.
 template <bool RECT, bool FAR>
